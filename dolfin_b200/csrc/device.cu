@@ -45,6 +45,36 @@ void DeviceBuffer::upload(const void* host, size_t nbytes) {
   if (e != cudaSuccess) fail(DB2_ERR_CUDA, "cudaMemcpy H2D: %s", cudaGetErrorString(e));
 }
 
+PlanUpload::PlanUpload() {
+  cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&m);
+  mode_ = int(m);
+  cudaStream_t s = nullptr;
+  const cudaError_t e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e != cudaSuccess) {
+    cudaThreadExchangeStreamCaptureMode(&m);
+    fail(DB2_ERR_CUDA, "plan stream: %s", cudaGetErrorString(e));
+  }
+  stream_ = s;
+}
+
+PlanUpload::~PlanUpload() {
+  cudaStream_t s = static_cast<cudaStream_t>(stream_);
+  cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  cudaStreamCaptureMode m = cudaStreamCaptureMode(mode_);
+  cudaThreadExchangeStreamCaptureMode(&m);
+}
+
+void PlanUpload::put(DeviceBuffer& d, const void* host, size_t nbytes) {
+  d.alloc(nbytes);
+  if (nbytes == 0) return;
+  cudaStream_t s = static_cast<cudaStream_t>(stream_);
+  cudaError_t e = cudaMemcpyAsync(d.ptr, host, nbytes, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the host array may go
+  if (e != cudaSuccess) fail(DB2_ERR_CUDA, "plan upload: %s", cudaGetErrorString(e));
+}
+
 // Vertex records of 4 doubles -- (x, y, z, kappa) in 3D, (x, y, kappa, f) in
 // 2D -- so that a vertex is one aligned 256-bit load; the coefficient slots
 // are written per assembly call (pack_vertex_records).

@@ -12,8 +12,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 #include <numeric>
-#include <thread>
 
 #include "internal.h"
 
@@ -36,25 +36,6 @@ int nedges(int tdim) { return tdim == 3 ? 6 : (tdim == 2 ? 3 : 0); }
 static const int kTetE[6][2] = {{2, 3}, {1, 3}, {1, 2}, {0, 3}, {0, 2}, {0, 1}};
 static const int kTriE[3][2] = {{1, 2}, {0, 2}, {0, 1}};
 static const int (*etab(int tdim))[2] { return tdim == 3 ? kTetE : kTriE; }
-
-// Run f(begin, end) over [0, n) on up to hardware_concurrency threads.
-template <typename F>
-static void parallel_for(int64_t n, F&& f, int64_t min_chunk = 4096) {
-  int nt = (int)std::max(1u, std::thread::hardware_concurrency());
-  nt = (int)std::min<int64_t>(nt, std::max<int64_t>(1, n / min_chunk));
-  if (nt <= 1) {
-    f((int64_t)0, n);
-    return;
-  }
-  std::vector<std::thread> th;
-  const int64_t chunk = (n + nt - 1) / nt;
-  for (int t = 0; t < nt; ++t) {
-    const int64_t b = t * chunk, e = std::min(n, b + chunk);
-    if (b >= e) break;
-    th.emplace_back([&f, b, e] { f(b, e); });
-  }
-  for (auto& t : th) t.join();
-}
 
 // ---------------------------------------------------------------------------
 // Meshes
@@ -622,13 +603,24 @@ std::shared_ptr<Pattern> make_pattern(std::shared_ptr<Space> V, bool keep_diagon
     buf.erase(std::unique(buf.begin(), buf.end()), buf.end());
   };
   std::atomic<int64_t> too_long{-1};
+  // the rows of each thread's range, joined once the row pointers are known
+  struct Rows {
+    int64_t begin;
+    std::vector<int32_t> cols;
+  };
+  std::vector<Rows> ranges;
+  std::mutex lock;
   parallel_for(nn, [&](int64_t b, int64_t e) {
     std::vector<uint32_t> buf;
+    Rows R{b, {}};
     for (int64_t i = b; i < e; ++i) {
       neighbours(i, buf);
       if (buf.size() > 255) too_long = i;
       P->node_rowptr[i + 1] = int32_t(buf.size());
+      R.cols.insert(R.cols.end(), buf.begin(), buf.end());
     }
+    std::lock_guard<std::mutex> g(lock);
+    ranges.push_back(std::move(R));
   });
   if (too_long >= 0) fail(DB2_ERR_UNSUPPORTED, "node %lld has more than 255 neighbours", (long long)too_long.load());
   int64_t acc = 0;
@@ -641,6 +633,12 @@ std::shared_ptr<Pattern> make_pattern(std::shared_ptr<Space> V, bool keep_diagon
   P->nnz = acc * P->bs * P->bs;
   P->nrows = nn * P->bs;
   P->node_cols.resize(acc);
+  parallel_for(int64_t(ranges.size()), [&](int64_t b, int64_t e) {
+    for (int64_t r = b; r < e; ++r) {
+      std::copy(ranges[r].cols.begin(), ranges[r].cols.end(), P->node_cols.begin() + P->node_rowptr[ranges[r].begin]);
+      std::vector<int32_t>().swap(ranges[r].cols);
+    }
+  }, 1);
 
   // column slots of each incidence's (relabelled) cell nodes
   P->kp = (k + 3) / 4 * 4;
@@ -648,17 +646,14 @@ std::shared_ptr<Pattern> make_pattern(std::shared_ptr<Space> V, bool keep_diagon
   std::vector<std::vector<int>> maps(k, std::vector<int>(k));
   for (int li = 0; li < k; ++li) canonical_node_map(m.tdim, V->degree, li, maps[li].data());
   parallel_for(nn, [&](int64_t b, int64_t e) {
-    std::vector<uint32_t> buf;
     for (int64_t i = b; i < e; ++i) {
-      neighbours(i, buf);
-      std::copy(buf.begin(), buf.end(), P->node_cols.begin() + P->node_rowptr[i]);
+      const int32_t* lo = P->node_cols.data() + P->node_rowptr[i];
+      const int32_t* hi = P->node_cols.data() + P->node_rowptr[i + 1];
       for (uint32_t s = P->inc_ptr[i]; s < P->inc_ptr[i + 1]; ++s) {
         const uint32_t c = P->inc[s] & 0x0fffffffu, li = P->inc[s] >> 28;
         const uint32_t* cn = &V->cell_nodes[int64_t(c) * k];
-        for (int j = 0; j < k; ++j) {
-          const uint32_t node = cn[maps[li][j]];
-          P->pos[int64_t(s) * P->kp + j] = uint8_t(std::lower_bound(buf.begin(), buf.end(), node) - buf.begin());
-        }
+        for (int j = 0; j < k; ++j)
+          P->pos[int64_t(s) * P->kp + j] = uint8_t(std::lower_bound(lo, hi, int32_t(cn[maps[li][j]])) - lo);
       }
     }
   });

@@ -1,9 +1,11 @@
 // internal.h -- host-side data structures of the engine (not part of the ABI).
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <memory>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/dolfin_b200.h"
@@ -17,6 +19,25 @@ struct Error {
 };
 [[noreturn]] void fail(int code, const char* fmt, ...);
 
+// Run f(begin, end) over [0, n) on up to hardware_concurrency threads.
+template <typename F>
+void parallel_for(int64_t n, F&& f, int64_t min_chunk = 4096) {
+  int nt = (int)std::max(1u, std::thread::hardware_concurrency());
+  nt = (int)std::min<int64_t>(nt, std::max<int64_t>(1, n / min_chunk));
+  if (nt <= 1) {
+    f((int64_t)0, n);
+    return;
+  }
+  std::vector<std::thread> th;
+  const int64_t chunk = (n + nt - 1) / nt;
+  for (int t = 0; t < nt; ++t) {
+    const int64_t b = t * chunk, e = std::min(n, b + chunk);
+    if (b >= e) break;
+    th.emplace_back([&f, b, e] { f(b, e); });
+  }
+  for (auto& t : th) t.join();
+}
+
 // Device buffer with RAII release (cudaFree); defined in device.cu.
 struct DeviceBuffer {
   void* ptr = nullptr;
@@ -28,6 +49,20 @@ struct DeviceBuffer {
   void alloc(size_t nbytes);
   void upload(const void* host, size_t nbytes);  // alloc + synchronous copy
   template <typename T> T* as() const { return static_cast<T*>(ptr); }
+};
+
+// Device work while a plan is built on first use, also when the caller's stream
+// is being captured into a graph: allocations and copies on a stream of their
+// own, outside the capture, complete when the scope ends.
+struct PlanUpload {
+  PlanUpload();
+  ~PlanUpload();
+  PlanUpload(const PlanUpload&) = delete;
+  PlanUpload& operator=(const PlanUpload&) = delete;
+  void put(DeviceBuffer& d, const void* host, size_t nbytes);  // alloc + copy
+ private:
+  void* stream_ = nullptr;
+  int mode_;
 };
 
 // ---- mesh ----------------------------------------------------------------
@@ -116,6 +151,43 @@ struct ReorderedCSR {
   DeviceBuffer d_vals, d_b, d_flags, d_bcv, d_vec;  // natural-order scratch
 };
 
+// Cell patches (patch_plan.cpp): the cells cut into compact clusters, one CTA
+// each, for what is summed per node over its cells (matrix-free action, load
+// vector).  A patch computes its cells' values in shared memory and sums them
+// per node there; a node whose cells all lie in the patch is finished, the
+// others leave one partial sum per patch, added up by a second kernel in
+// patch order.  So a cell's values never reach HBM.
+struct PatchHdr {
+  uint32_t cell0, node0;       // first cell / local node in the plan's arrays
+  uint32_t chunk0, chunks;     // jobs: first 16-byte unit, and how many
+  uint16_t ncells, nnodes, nverts, ngroups;
+  uint32_t pad[2];
+};
+// 32 node sums, one per lane: values codes[code0 + 32 t + lane], t < width, of
+// the patch's staged values (8 (local node * stride + cell)), in ascending cell
+// order; shorter sums are padded with the zero slot.
+struct PatchGroup {
+  uint32_t code0;
+  uint16_t width, live;
+};
+constexpr int patch_conn(int k) { return (k + 3) / 4 * 4; }  // entries of a cell
+constexpr uint32_t kPatchPartial = 1u << 31;  // destination: a partial slot, else a node
+struct PatchPlan {
+  int stride = 0;              // cells of the largest patch, odd
+  int max_nodes = 0, max_verts = 0, max_chunks = 0;
+  int64_t npatches = 0, nshared = 0, npartial = 0;
+  std::vector<PatchHdr> hdr;
+  std::vector<uint32_t> nodes;   // global ids of the patch's nodes, ascending
+  // per cell: 8 x its local nodes (byte offsets of doubles), padded to 8 bytes
+  std::vector<uint16_t> conn;
+  std::vector<uint8_t> chunks;   // per patch: destinations (32 a group), groups, codes
+  std::vector<uint32_t> shared;  // nodes with partial sums
+  std::vector<uint32_t> shared_ptr;  // their partial slots, in patch order
+  DeviceBuffer d_hdr, d_conn, d_nodes, d_chunks, d_shared, d_shared_ptr, d_partial;
+  DeviceBuffer d_x;              // copy of an x that shares memory with y
+  static constexpr uint32_t pad16(uint32_t n) { return (n + 15u) & ~15u; }
+};
+
 struct Pattern {
   std::shared_ptr<Space> V;
   bool keep_diagonal = false;
@@ -158,8 +230,7 @@ struct Pattern {
   // each node's first record again, node-indexed: the row walk's first
   // record load needs no rec_goff lookup before it
   DeviceBuffer d_rec_first;
-  // matrix-free action: per-cell element actions (cells x bs x k), grown on
-  // first use
+  // tensor-core action: per-cell element actions, grown on first use
   mutable DeviceBuffer d_cellvals;
   bool on_device = false;
   void ensure_device();      // first GPU use: upload the plan, expand the CSR
@@ -170,6 +241,7 @@ struct Pattern {
   ReorderedCSR reordered;
   std::unique_ptr<FacetPlan> facets;
   const FacetPlan& facet_plan();     // built and uploaded on first use
+  mutable std::unique_ptr<PatchPlan> patches;
 };
 
 // Relabelling of a cell so that local node `li` becomes canonical: for a
@@ -201,6 +273,10 @@ int64_t read_vector_xml(const char* path, double* x, int64_t cap);  // x NULL: s
 // Host-side facet plan of a pattern (no device work); Pattern::facet_plan()
 // also uploads it.
 void build_facet_plan(Pattern& P);
+// Cell patches of a pattern (host side), of at most max_cells cells.
+std::unique_ptr<PatchPlan> make_patches(const Pattern& P, int max_cells);
+// The pattern's patches, built and uploaded on first use.
+const PatchPlan& patch_plan(const Pattern& P);
 // Re-cut the tiles of an existing plan (autotuning), re-uploading d_tiles.
 void retile(Pattern& P, int tile_threads, int seg_cap_bytes);
 // Tiles of a pattern for a launch shape (pure; does not modify P).

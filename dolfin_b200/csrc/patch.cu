@@ -1,0 +1,515 @@
+// patch.cu -- matrix-free action y = A x over cell patches (PatchPlan): a CTA
+// per patch stages its nodes' x and its vertices' coordinates in shared
+// memory, a thread per cell computes the cell's action y_K = A_K x_K into
+// shared memory, and the patch's nodes sum their cells there in ascending cell
+// order.  Nodes shared between patches leave a partial sum per patch, added
+// in patch order by a second kernel.  The order of additions is fixed, so the
+// result is bitwise repeatable.
+//
+// Against writing every cell's action to HBM and gathering it per row (2 x 8
+// bytes per cell and local node, 0.85 GB at P2 n=96), a patch moves its plan
+// (60 B a cell), x, y and about one partial sum a cell.  Measured on B200, ms
+// per action: vector P2 elasticity n=48 0.245 -> 0.087, P2 tets n=96 0.342 ->
+// 0.230, P1 tets n=80 0.102 -> 0.060; with FP32 actions 63x70x57 0.084 ->
+// 0.081 (its quadrature is unchanged, and issue-bound).
+#include <cuda_runtime.h>
+
+#include "launch.cuh"
+#include "quad.cuh"
+
+namespace db2 {
+namespace dev {
+
+struct PatchArgs {
+  const PatchHdr* hdr;
+  const uint16_t* conn;
+  const uint32_t* nodes;
+  const uint4* chunks;
+  const double* xw;     // vertex records, coordinates first
+  const double* kappa;  // P1 field or null
+  double kscale, mu, lmbda;
+  const double* x;
+  double* y;
+  double* partial;
+  int64_t nnodes, npartial;
+  int stride;           // staged cells of a local node
+  int nx, nv;           // room for the patch's nodes and vertices
+  uint32_t ahead;       // patches in flight on the device
+};
+
+__device__ __forceinline__ PatchHdr patch_header(const PatchHdr* hdr, uint32_t i) {
+  const uint4* s = reinterpret_cast<const uint4*>(hdr + i);
+  const uint4 a = __ldg(s), b = __ldg(s + 1);
+  PatchHdr h;
+  h.cell0 = a.x;
+  h.node0 = a.y;
+  h.chunk0 = a.z;
+  h.chunks = a.w;
+  h.ncells = uint16_t(b.x & 0xffffu);
+  h.nnodes = uint16_t(b.x >> 16);
+  h.nverts = uint16_t(b.y & 0xffffu);
+  h.ngroups = uint16_t(b.y >> 16);
+  return h;
+}
+
+// Element action of P2 by exact moments, FP64.  With U_m the gradient of u at
+// vertex m (grad u is linear), F the flux and M_m = int lambda_m F:
+//   y_v = g_v . (4 M_v - sum_m M_m),   y_(p,q) = 4 (g_p . M_q + g_q . M_p),
+// where for a linear flux (F_m its vertex values) M_m = |T| c2 (sum F + F_m),
+// and for F = kappa grad u with linear kappa, by int lambda_m lambda_k lambda_l,
+//   M_m = |T| c3 [(sum kappa)(sum U) + sum kappa_k U_k + kappa_m (sum U + 2 U_m)
+//                 + (sum kappa) U_m].
+// About half the operations of the quadrature of the same degree (P2
+// tetrahedra, linear kappa: ~230 against ~430).
+template <int D>
+constexpr double moment2() { return D == 3 ? 1.0 / 20 : 1.0 / 12; }
+template <int D>
+constexpr double moment3() { return D == 3 ? 1.0 / 120 : 1.0 / 60; }
+
+// Gradients of one P2 component at the vertices: U_m = sum_a d_a g_a with
+// d_a = 4 x_(a,m) - x_a (a != m), 3 x_m (a = m).
+template <int D>
+__device__ __forceinline__ void p2_vertex_gradients(const double (&xc)[El<D, 2>::K], const double (&g)[D + 1][D],
+                                                    double (&U)[D + 1][D]) {
+#pragma unroll
+  for (int m = 0; m <= D; ++m) {
+#pragma unroll
+    for (int r = 0; r < D; ++r) U[m][r] = 0.0;
+#pragma unroll
+    for (int a = 0; a <= D; ++a) {
+      const double d = a == m ? 3.0 * xc[m] : fma(4.0, xc[D + 1 + cell_edge_of(D, a, m)], -xc[a]);
+#pragma unroll
+      for (int r = 0; r < D; ++r) U[m][r] = fma(d, g[a][r], U[m][r]);
+    }
+  }
+}
+
+template <int D>
+__device__ __forceinline__ double dotg(const double (&a)[D], const double (&b)[D]) {
+  double s = a[0] * b[0];
+#pragma unroll
+  for (int r = 1; r < D; ++r) s = fma(a[r], b[r], s);
+  return s;
+}
+
+// P2 test functions against the moments M and t_v = 4 M_v - sum M.
+template <int D>
+__device__ __forceinline__ void p2_test(const double (&M)[D + 1][D], const double (&t)[D + 1][D],
+                                        const double (&g)[D + 1][D], double (&y)[El<D, 2>::K]) {
+#pragma unroll
+  for (int v = 0; v <= D; ++v) y[v] = dotg<D>(g[v], t[v]);
+#pragma unroll
+  for (int e = 0; e < El<D, 2>::NE; ++e) {
+    const int p = edge_end(D, e, 0), q = edge_end(D, e, 1);
+    double s = dotg<D>(g[p], M[q]);
+#pragma unroll
+    for (int r = 0; r < D; ++r) s = fma(g[q][r], M[p][r], s);
+    y[D + 1 + e] = 4.0 * s;
+  }
+}
+
+// A linear flux of vertex values F: M_m = S + F_m with S = sum F (times |T|
+// c2), so t_v = 4 F_v - (D - 2) S.
+template <int D>
+__device__ __forceinline__ void p2_test_linear(const double (&F)[D + 1][D], const double (&g)[D + 1][D],
+                                               double (&y)[El<D, 2>::K]) {
+  double M[D + 1][D], t[D + 1][D];
+#pragma unroll
+  for (int r = 0; r < D; ++r) {
+    double S = F[0][r];
+#pragma unroll
+    for (int m = 1; m <= D; ++m) S += F[m][r];
+#pragma unroll
+    for (int m = 0; m <= D; ++m) {
+      M[m][r] = S + F[m][r];
+      t[m][r] = D == 3 ? fma(4.0, F[m][r], -S) : 4.0 * F[m][r];
+    }
+  }
+  p2_test<D>(M, t, g, y);
+}
+
+// y_K = A_K x_K of one cell, every component.
+template <int D, int P, int FORM, bool KP1, typename CT>
+__device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&xv)[D + 1][D],
+                                            const double (&kap)[D + 1],
+                                            const double (&xc)[FORM == FORM_ELAS ? D : 1][El<D, P>::K],
+                                            double (&y)[FORM == FORM_ELAS ? D : 1][El<D, P>::K]) {
+  constexpr int NB = D + 1, K = El<D, P>::K, BS = FORM == FORM_ELAS ? D : 1;
+  double g[NB][D];
+  const double vol = bary_gradients<D>(xv, g);
+  if constexpr (P == 2 && sizeof(CT) == 8) {
+    if constexpr (FORM == FORM_DIFF) {
+      double U[NB][D];
+      p2_vertex_gradients<D>(xc[0], g, U);
+      const double w = vol * q.kscale * (KP1 ? moment3<D>() : moment2<D>());
+      if constexpr (KP1) {
+        double M[NB][D], t[NB][D];
+        double sk = kap[0];
+#pragma unroll
+        for (int m = 1; m <= D; ++m) sk += kap[m];
+#pragma unroll
+        for (int r = 0; r < D; ++r) {
+          double SU = U[0][r];
+#pragma unroll
+          for (int m = 1; m <= D; ++m) SU += U[m][r];
+          double base = sk * SU;
+#pragma unroll
+          for (int m = 0; m <= D; ++m) base = fma(kap[m], U[m][r], base);
+          double M0 = 0.0;
+#pragma unroll
+          for (int m = 0; m <= D; ++m) {
+            M[m][r] = w * fma(sk, U[m][r], fma(kap[m], fma(2.0, U[m][r], SU), base));
+            M0 += M[m][r];
+          }
+#pragma unroll
+          for (int m = 0; m <= D; ++m) t[m][r] = fma(4.0, M[m][r], -M0);
+        }
+        p2_test<D>(M, t, g, y[0]);
+      } else {
+#pragma unroll
+        for (int m = 0; m <= D; ++m)
+#pragma unroll
+          for (int r = 0; r < D; ++r) U[m][r] *= w;
+        p2_test_linear<D>(U, g, y[0]);
+      }
+    } else {
+      // stress at the vertices: lambda div(u) I + mu (grad u + grad u^T)
+      double sg[NB][D][D];
+#pragma unroll
+      for (int e = 0; e < D; ++e) {
+        double U[NB][D];
+        p2_vertex_gradients<D>(xc[e], g, U);
+#pragma unroll
+        for (int m = 0; m <= D; ++m)
+#pragma unroll
+          for (int d = 0; d < D; ++d) sg[m][e][d] = U[m][d];
+      }
+      const double w = vol * moment2<D>();
+#pragma unroll
+      for (int m = 0; m <= D; ++m) {
+        double div = sg[m][0][0];
+#pragma unroll
+        for (int d = 1; d < D; ++d) div += sg[m][d][d];
+        const double l = w * q.lmbda * div, mu = w * q.mu;
+#pragma unroll
+        for (int c = 0; c < D; ++c)
+#pragma unroll
+          for (int d = c; d < D; ++d) {
+            const double s = mu * (sg[m][c][d] + sg[m][d][c]) + (c == d ? l : 0.0);
+            sg[m][c][d] = sg[m][d][c] = s;
+          }
+      }
+#pragma unroll
+      for (int c = 0; c < D; ++c) {
+        double F[NB][D];
+#pragma unroll
+        for (int m = 0; m <= D; ++m)
+#pragma unroll
+          for (int d = 0; d < D; ++d) F[m][d] = sg[m][c][d];
+        p2_test_linear<D>(F, g, y[c]);
+      }
+    }
+  } else {
+    // quadrature (P1: the centroid), in the contraction type
+    using Q = Quad<D, P == 1 ? 1 : (FORM == FORM_ELAS ? 2 : 3)>;
+    CT gc[NB][D], xq[BS][K];
+#pragma unroll
+    for (int a = 0; a < NB; ++a)
+#pragma unroll
+      for (int r = 0; r < D; ++r) gc[a][r] = CT(g[a][r]);
+#pragma unroll
+    for (int e = 0; e < BS; ++e)
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        xq[e][j] = CT(xc[e][j]);
+        y[e][j] = 0.0;
+      }
+#pragma unroll
+    for (int n = 0; n < Q::NQ; ++n) {
+      double l[NB];
+#pragma unroll
+      for (int a = 0; a < NB; ++a) l[a] = Q::lam(n, a);
+      const double wq = Q::w(n) * vol;
+      CT gu[BS][D];
+#pragma unroll
+      for (int e = 0; e < BS; ++e) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) gu[e][d] = CT(0);
+#pragma unroll
+        for (int a = 0; a < NB; ++a) {
+          const CT u = node_derivative<D, P, CT>(xq[e], l, a);
+#pragma unroll
+          for (int d = 0; d < D; ++d) gu[e][d] = fma(u, gc[a][d], gu[e][d]);
+        }
+      }
+#pragma unroll
+      for (int c = 0; c < BS; ++c) {
+        CT flux[D];
+        if constexpr (FORM == FORM_ELAS) {
+          CT div = gu[0][0];
+#pragma unroll
+          for (int d = 1; d < D; ++d) div += gu[d][d];
+#pragma unroll
+          for (int d = 0; d < D; ++d) flux[d] = CT(q.mu) * (gu[c][d] + gu[d][c]);
+          flux[c] = fma(CT(q.lmbda), div, flux[c]);
+        } else {
+          double k = q.kscale;
+          if constexpr (KP1) {
+            double kq = 0.0;
+#pragma unroll
+            for (int a = 0; a < NB; ++a) kq = fma(kap[a], l[a], kq);
+            k *= kq;
+          }
+#pragma unroll
+          for (int d = 0; d < D; ++d) flux[d] = CT(k) * gu[0][d];
+        }
+        CT S[NB];
+#pragma unroll
+        for (int a = 0; a < NB; ++a) {
+          CT sa = flux[0] * gc[a][0];
+#pragma unroll
+          for (int d = 1; d < D; ++d) sa = fma(flux[d], gc[a][d], sa);
+          S[a] = CT(wq) * sa;
+        }
+        test_basis<D, P, CT>(S, l, y[c]);
+      }
+    }
+  }
+}
+
+// Block size and CTAs per SM.  The kernel is bound by latency -- the plan's and
+// x's loads at a CTA's start, then dependent shared-memory reads and FP64
+// chains -- so small blocks, many of them resident, win.  P2 tets n=96, ms per
+// action: 128 threads, five CTAs (96 registers) 0.246; four 0.280; six (80
+// registers, spills) 0.295; 96 threads 0.346; 192 threads 0.32-0.35; 256
+// threads 0.53.  Elasticity takes 126 registers and four CTAs: 0.089 against
+// 0.13 (five) and 0.18 (six).
+constexpr int kPatchThreads = 128;
+template <int FORM>
+constexpr int patch_ctas() {
+  return FORM == FORM_ELAS ? 4 : 5;
+}
+template <int D, int P, int FORM, bool KP1, typename CT>
+__global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_apply(const PatchArgs q) {
+  constexpr int NB = D + 1, K = El<D, P>::K, BS = FORM == FORM_ELAS ? D : 1;
+  constexpr int T = kPatchThreads;
+  extern __shared__ __align__(16) unsigned char smem[];
+  // the nodes' x by component, vertex records (x, y, z, kappa), the staged
+  // actions by component and local node (and a zero slot each), the jobs
+  double* xs = reinterpret_cast<double*>(smem);
+  double* vs = xs + BS * q.nx;
+  CT* ys = reinterpret_cast<CT*>(vs + 4 * q.nv);
+  const int plane = K * q.stride + 1;
+  unsigned char* jobs = smem + PatchPlan::pad16(uint32_t((4 * q.nv + BS * q.nx) * 8 + BS * plane * int(sizeof(CT))));
+  const PatchHdr h = patch_header(q.hdr, blockIdx.x);
+  // the plan data of a patch that starts later goes to L2 meanwhile (P2 tets
+  // n=96 0.246 -> 0.230 ms)
+  const uint32_t later = blockIdx.x + q.ahead;
+  PatchHdr hn{};
+  if (later < gridDim.x) hn = patch_header(q.hdr, later);
+  {
+    const uint4* src = q.chunks + h.chunk0;
+    const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(jobs));
+    for (uint32_t i = threadIdx.x; i < h.chunks; i += T)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16u * i), "l"(src + i) : "memory");
+  }
+  // the cells' local nodes are loaded one cell ahead
+  constexpr int KC = patch_conn(K) / 4;
+  const uint2* conn = reinterpret_cast<const uint2*>(q.conn) + size_t(h.cell0) * KC;
+  uint2 cn[KC];
+#pragma unroll
+  for (int i = 0; i < KC; ++i)
+    cn[i] = int(threadIdx.x) < h.ncells ? __ldg(conn + threadIdx.x * KC + i) : make_uint2(0u, 0u);
+  for (int i = threadIdx.x; i < h.nnodes; i += T) {
+    const uint32_t node = __ldg(q.nodes + h.node0 + i);
+#pragma unroll
+    for (int e = 0; e < BS; ++e) xs[e * q.nx + i] = __ldg(q.x + int64_t(e) * q.nnodes + node);
+    if (i < h.nverts) {
+      double a, b, c, d;
+      ld_rec4(q.xw + 4 * size_t(node), a, b, c, d);
+      double2* v = reinterpret_cast<double2*>(vs + 4 * i);
+      v[0] = make_double2(a, b);
+      v[1] = make_double2(D == 3 ? c : 0.0, KP1 ? __ldg(q.kappa + node) : 0.0);
+    }
+  }
+  if (threadIdx.x < BS) ys[threadIdx.x * plane + K * q.stride] = CT(0);
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  if (later < gridDim.x) {
+    auto prefetch = [](const void* p, uint32_t bytes) {
+      const char* b = static_cast<const char*>(p);
+      for (uint32_t i = 128u * threadIdx.x; i < bytes; i += 128u * T)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(b + i));
+    };
+    prefetch(q.nodes + hn.node0, hn.nnodes * 4u);
+    prefetch(reinterpret_cast<const uint2*>(q.conn) + size_t(hn.cell0) * KC, hn.ncells * KC * 8u);
+    prefetch(q.chunks + hn.chunk0, hn.chunks * 16u);
+  }
+  for (int c = threadIdx.x; c < h.ncells; c += T) {
+    double xv[NB][D], kap[NB], xc[BS][K], y[BS][K];
+    auto off = [&](int j) {  // 8 x local node j
+      const uint32_t w = (j & 2) ? cn[j >> 2].y : cn[j >> 2].x;
+      return (j & 1) ? w >> 16 : w & 0xffffu;
+    };
+#pragma unroll
+    for (int a = 0; a < NB; ++a) {
+      const double2* v = reinterpret_cast<const double2*>(reinterpret_cast<const char*>(vs) + 4 * off(a));
+      const double2 lo = v[0], hi = v[1];
+      xv[a][0] = lo.x;
+      xv[a][1] = lo.y;
+      if constexpr (D == 3) xv[a][2] = hi.x;
+      kap[a] = hi.y;
+    }
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      const char* xj = reinterpret_cast<const char*>(xs) + off(j);
+#pragma unroll
+      for (int e = 0; e < BS; ++e) xc[e][j] = reinterpret_cast<const double*>(xj)[e * q.nx];
+    }
+    if (c + T < h.ncells) {
+#pragma unroll
+      for (int i = 0; i < KC; ++i) cn[i] = __ldg(conn + (c + T) * KC + i);
+    }
+    cell_action<D, P, FORM, KP1, CT>(q, xv, kap, xc, y);
+#pragma unroll
+    for (int e = 0; e < BS; ++e)
+#pragma unroll
+      for (int j = 0; j < K; ++j) ys[e * plane + j * q.stride + c] = CT(y[e][j]);
+  }
+  __syncthreads();
+  const uint32_t* dest = reinterpret_cast<const uint32_t*>(jobs);
+  const PatchGroup* groups = reinterpret_cast<const PatchGroup*>(jobs + 128u * h.ngroups);
+  const uint16_t* codes = reinterpret_cast<const uint16_t*>(
+      jobs + 128u * h.ngroups + PatchPlan::pad16(h.ngroups * uint32_t(sizeof(PatchGroup))));
+  const int lane = threadIdx.x & 31;
+  for (int g = threadIdx.x >> 5; g < h.ngroups; g += T / 32) {
+    const PatchGroup gr = groups[g];
+    const uint16_t* code = codes + gr.code0 + lane;
+    double acc[BS];
+#pragma unroll
+    for (int e = 0; e < BS; ++e) acc[e] = 0.0;
+#pragma unroll 4
+    for (int t = 0; t < gr.width; ++t) {
+      const uint32_t w = sizeof(CT) == 8 ? code[32 * t] : code[32 * t] / 2u;
+      const CT* v = reinterpret_cast<const CT*>(reinterpret_cast<const char*>(ys) + w);
+#pragma unroll
+      for (int e = 0; e < BS; ++e) acc[e] += double(v[e * plane]);
+    }
+    if (lane < gr.live) {
+      const uint32_t d = dest[32 * g + lane];
+      double* out = d & kPatchPartial ? q.partial + (d & ~kPatchPartial) : q.y + d;
+      const int64_t step = d & kPatchPartial ? q.npartial : q.nnodes;
+#pragma unroll
+      for (int e = 0; e < BS; ++e) out[e * step] = acc[e];
+    }
+  }
+}
+
+// Nodes shared between patches: their partial sums in patch order.
+template <int BS>
+__global__ void __launch_bounds__(256) k_patch_sum(const uint32_t* __restrict__ shared,
+                                                   const uint32_t* __restrict__ ptr, int64_t n,
+                                                   const double* __restrict__ partial, int64_t npartial,
+                                                   double* __restrict__ y, int64_t nnodes) {
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const uint32_t node = __ldg(shared + i), s0 = __ldg(ptr + i), s1 = __ldg(ptr + i + 1);
+  double acc[BS];
+#pragma unroll
+  for (int e = 0; e < BS; ++e) acc[e] = 0.0;
+  for (uint32_t s = s0; s < s1; ++s)
+#pragma unroll
+    for (int e = 0; e < BS; ++e) acc[e] += __ldg(partial + int64_t(e) * npartial + s);
+#pragma unroll
+  for (int e = 0; e < BS; ++e) y[int64_t(e) * nnodes + node] = acc[e];
+}
+
+template <int D, int P, int FORM, bool KP1, typename CT>
+void run_patch_apply(const PatchPlan& B, PatchArgs q, cudaStream_t s) {
+  constexpr int K = El<D, P>::K, BS = FORM == FORM_ELAS ? D : 1;
+  if (B.npatches > 0) {
+    auto kern = k_patch_apply<D, P, FORM, KP1, CT>;
+    static unsigned long long configured = 0;
+    allow_dynamic_smem(kern, configured);
+    const size_t smem = PatchPlan::pad16(uint32_t((4 * q.nv + BS * q.nx) * 8 + BS * (K * q.stride + 1) * int(sizeof(CT)))) +
+                        size_t(B.max_chunks) * 16;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    q.ahead = uint32_t(sms * patch_ctas<FORM>());
+    kern<<<unsigned(B.npatches), kPatchThreads, smem, s>>>(q);
+    count_launch();
+    check_cuda("patch apply launch");
+  }
+  if (B.nshared > 0) {
+    k_patch_sum<BS><<<unsigned((B.nshared + 255) / 256), 256, 0, s>>>(B.d_shared.as<uint32_t>(), B.d_shared_ptr.as<uint32_t>(),
+                                                                      B.nshared, q.partial, B.npartial, q.y, q.nnodes);
+    count_launch();
+    check_cuda("patch sum launch");
+  }
+}
+
+}  // namespace dev
+
+void launch_patch_apply(const Pattern& P, const dev::AsmParams& p, bool elas, bool kp1, bool fp32, const double* x,
+                        double* y, void* stream) {
+  const PatchPlan& B = patch_plan(P);
+  dev::PatchArgs q{};
+  q.hdr = B.d_hdr.as<PatchHdr>();
+  q.conn = B.d_conn.as<uint16_t>();
+  q.nodes = B.d_nodes.as<uint32_t>();
+  q.chunks = B.d_chunks.as<uint4>();
+  q.xw = p.xw;
+  q.kappa = kp1 ? p.kappa : nullptr;
+  q.kscale = p.kscale;
+  q.mu = p.mu;
+  q.lmbda = p.lmbda;
+  const int64_t n = P.V->dim();
+  cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // a patch writes its finished nodes while others still read x: an x that
+  // shares memory with y is copied first
+  if (x < y + n && y < x + n) {
+    DeviceBuffer& c = const_cast<PatchPlan&>(B).d_x;
+    if (c.bytes < size_t(n) * sizeof(double)) {
+      PlanUpload scope;
+      c.alloc(size_t(n) * sizeof(double));
+    }
+    cudaMemcpyAsync(c.ptr, x, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
+    check_cuda("copy of x");
+    x = c.as<double>();
+  }
+  q.x = x;
+  q.y = y;
+  q.partial = B.d_partial.as<double>();
+  q.nnodes = p.nnodes;
+  q.npartial = B.npartial;
+  q.stride = B.stride;
+  q.nx = (B.max_nodes + 1) & ~1;  // (the vertex records behind start on 16 bytes)
+  q.nv = B.max_verts;
+  const int D = P.V->mesh->tdim, deg = P.V->degree;
+  if (elas) {
+    if (deg == 1) {
+      if (fp32) dev::run_patch_apply<3, 1, dev::FORM_ELAS, false, float>(B, q, s);
+      else dev::run_patch_apply<3, 1, dev::FORM_ELAS, false, double>(B, q, s);
+    } else {
+      if (fp32) dev::run_patch_apply<3, 2, dev::FORM_ELAS, false, float>(B, q, s);
+      else dev::run_patch_apply<3, 2, dev::FORM_ELAS, false, double>(B, q, s);
+    }
+    return;
+  }
+#define DB2_PA(D_, P_)                                                                   \
+  if (D == D_ && deg == P_) {                                                            \
+    if (kp1) {                                                                           \
+      if (fp32) dev::run_patch_apply<D_, P_, dev::FORM_DIFF, true, float>(B, q, s);      \
+      else dev::run_patch_apply<D_, P_, dev::FORM_DIFF, true, double>(B, q, s);          \
+    } else {                                                                             \
+      if (fp32) dev::run_patch_apply<D_, P_, dev::FORM_DIFF, false, float>(B, q, s);     \
+      else dev::run_patch_apply<D_, P_, dev::FORM_DIFF, false, double>(B, q, s);         \
+    }                                                                                    \
+    return;                                                                              \
+  }
+  DB2_PA(3, 1) DB2_PA(3, 2) DB2_PA(2, 1) DB2_PA(2, 2)
+#undef DB2_PA
+}
+
+}  // namespace db2

@@ -1,0 +1,362 @@
+// patch_plan.cpp -- cell patches of a pattern (PatchPlan, internal.h).
+//
+// A cell belongs to its first vertex; the vertices are clustered by recursive
+// bisection of their coordinates along the longest side, cut at the widest gap
+// near the position that fills the patches.  On lattice-like meshes (jittered ones too) the cuts fall
+// between lattice planes and patches are boxes, with few nodes shared between
+// them; elsewhere they are cut at that position.
+#include <cmath>
+#include <cstring>
+#include <numeric>
+
+#include "internal.h"
+
+namespace db2 {
+namespace {
+
+struct Bisector {
+  const Mesh& m;
+  const std::vector<uint32_t>& cell0;  // first cell (by first vertex) of each vertex
+  int max_cells;
+
+  int64_t cells_of(const uint32_t* v, int64_t n) const {
+    int64_t c = 0;
+    for (int64_t i = 0; i < n; ++i) c += cell0[v[i] + 1] - cell0[v[i]];
+    return c;
+  }
+  // Reorders v[0, n), n > 1, and returns the cut (0 < cut < n): as many full
+  // patches on one side as on the other, or one more.
+  int64_t split(uint32_t* v, int64_t n) const {
+    const int D = m.tdim;
+    double lo[3], hi[3];
+    for (int r = 0; r < D; ++r) lo[r] = hi[r] = m.x[int64_t(v[0]) * D + r];
+    for (int64_t i = 1; i < n; ++i)
+      for (int r = 0; r < D; ++r) {
+        const double x = m.x[int64_t(v[i]) * D + r];
+        lo[r] = std::min(lo[r], x);
+        hi[r] = std::max(hi[r], x);
+      }
+    int axis = 0;
+    for (int r = 1; r < D; ++r)
+      if (hi[r] - lo[r] > hi[axis] - lo[axis]) axis = r;
+    auto key = [&](uint32_t a) { return m.x[int64_t(a) * D + axis]; };
+    auto less = [&](uint32_t a, uint32_t b) {
+      const double p = key(a), q = key(b);
+      return p < q || (!(q < p) && a < b);
+    };
+    const int64_t parts = (cells_of(v, n) + max_cells - 1) / max_cells;
+    const int64_t mid = std::min(n - 1, std::max<int64_t>(1, parts > 1 ? n * (parts / 2) / parts : n / 2));
+    // the window around it in which the cut may lie
+    // (about one lattice plane of n vertices to either side)
+    const int64_t w = std::max<int64_t>(1, std::min<int64_t>(n / 6, int64_t(std::pow(double(n), 2.0 / 3.0))));
+    const int64_t b = std::max<int64_t>(1, mid - w), e = std::min<int64_t>(n - 1, mid + w);
+    if (b >= e) {
+      std::nth_element(v, v + mid, v + n, less);
+      return mid;
+    }
+    std::nth_element(v, v + (b - 1), v + n, less);
+    std::nth_element(v + b, v + e, v + n, less);
+    std::sort(v + b, v + e, less);  // v[b - 1 .. e] now ascending
+    int64_t cut = mid;
+    double best = -1.0;
+    for (int64_t i = b; i <= e; ++i) {
+      const double gap = key(v[i]) - key(v[i - 1]);
+      const int64_t d = std::abs(i - mid), dc = std::abs(cut - mid);
+      if (gap > best * 1.5 || (gap > best / 1.5 && d < dc)) {
+        best = std::max(gap, best);
+        cut = i;
+      }
+    }
+    return cut;
+  }
+  void leaves(uint32_t* v, int64_t base, int64_t n, std::vector<int64_t>& ends) const {
+    if (n <= 1 || cells_of(v, n) <= max_cells) {
+      ends.push_back(base + n);
+      return;
+    }
+    const int64_t c = split(v, n);
+    leaves(v, base, c, ends);
+    leaves(v + c, base + c, n - c, ends);
+  }
+};
+
+// Node id -> local number, for one patch at a time (open addressing; clearing
+// is a new stamp).
+struct NodeTable {
+  std::vector<uint32_t> key, stamp, val;
+  uint32_t now = 0, mask;
+  explicit NodeTable(size_t nodes) {
+    size_t n = 64;
+    while (n < 2 * nodes) n *= 2;
+    key.resize(n);
+    stamp.assign(n, 0);
+    val.resize(n);
+    mask = uint32_t(n - 1);
+  }
+  void clear() { ++now; }
+  size_t find(uint32_t k) const {
+    size_t i = (k * 2654435761u >> 7) & mask;
+    while (stamp[i] == now && key[i] != k) i = (i + 1) & mask;
+    return i;
+  }
+  bool insert(uint32_t k) {  // true if it was not there
+    const size_t i = find(k);
+    if (stamp[i] == now) return false;
+    stamp[i] = now;
+    key[i] = k;
+    return true;
+  }
+};
+
+struct Part {  // patches of a contiguous range of clusters
+  std::vector<PatchHdr> hdr;
+  std::vector<uint32_t> cells;  // of each patch, ascending
+  std::vector<uint32_t> nodes;
+  std::vector<uint16_t> conn;
+  std::vector<uint8_t> chunks;
+  int max_nodes = 0, max_verts = 0, max_chunks = 0;
+};
+
+}  // namespace
+
+std::unique_ptr<PatchPlan> make_patches(const Pattern& P, int max_cells) {
+  const Space& V = *P.V;
+  const Mesh& m = *V.mesh;
+  const int k = V.k, nvc = m.tdim + 1, kc = patch_conn(k);
+  auto B = std::make_unique<PatchPlan>();
+  // 16-bit byte offsets of the staged values and of the local nodes
+  max_cells = std::min(max_cells, 8191 / k - 1);
+  if (uint64_t(V.nnodes) >= kPatchPartial) fail(DB2_ERR_UNSUPPORTED, "too many nodes for cell patches");
+  // cells by first vertex, ascending
+  std::vector<uint32_t> cell0(size_t(m.nv) + 1, 0), bucket(static_cast<size_t>(m.nc));
+  for (int64_t c = 0; c < m.nc; ++c) cell0[m.cells[c * nvc] + 1]++;
+  for (int64_t v = 0; v < m.nv; ++v) cell0[v + 1] += cell0[v];
+  {
+    std::vector<uint32_t> fill(cell0.begin(), cell0.end() - 1);
+    for (int64_t c = 0; c < m.nc; ++c) bucket[fill[m.cells[c * nvc]]++] = uint32_t(c);
+  }
+  std::vector<uint32_t> vert;
+  for (int64_t v = 0; v < m.nv; ++v)
+    if (cell0[v + 1] > cell0[v]) vert.push_back(uint32_t(v));
+  const Bisector C{m, cell0, max_cells};
+  // top levels of the bisection, then the parts in parallel
+  std::vector<int64_t> cuts{0, int64_t(vert.size())};
+  while (cuts.size() < 256 && m.nc / int64_t(cuts.size()) > 8 * max_cells) {
+    std::vector<int64_t> mid(cuts.size() - 1), next{0};
+    parallel_for(int64_t(mid.size()), [&](int64_t b, int64_t e) {
+      for (int64_t i = b; i < e; ++i) {
+        const int64_t n = cuts[i + 1] - cuts[i];
+        mid[i] = cuts[i] + (n > 1 ? C.split(vert.data() + cuts[i], n) : 0);
+      }
+    }, 1);
+    for (size_t i = 0; i + 1 < cuts.size(); ++i) {
+      if (mid[i] > cuts[i]) next.push_back(mid[i]);
+      next.push_back(cuts[i + 1]);
+    }
+    if (next.size() == cuts.size()) break;
+    cuts.swap(next);
+  }
+  const int64_t nparts = int64_t(cuts.size()) - 1;
+  std::vector<Part> parts(static_cast<size_t>(nparts));
+  // pass 1: the patches' cells and nodes
+  parallel_for(nparts, [&](int64_t b, int64_t e) {
+    std::vector<int64_t> ends;
+    std::vector<uint32_t> cells;
+    NodeTable table(size_t(max_cells) * k);
+    for (int64_t i = b; i < e; ++i) {
+      Part& T = parts[i];
+      ends.clear();
+      C.leaves(vert.data() + cuts[i], cuts[i], cuts[i + 1] - cuts[i], ends);
+      int64_t at = cuts[i];
+      for (int64_t end : ends) {
+        cells.clear();
+        for (; at < end; ++at)
+          cells.insert(cells.end(), bucket.begin() + cell0[vert[at]], bucket.begin() + cell0[vert[at] + 1]);
+        std::sort(cells.begin(), cells.end());
+        // (one vertex with more cells than a patch takes: several patches)
+        for (size_t c = 0; c < cells.size(); c += max_cells) {
+          const size_t n = std::min(cells.size() - c, size_t(max_cells));
+          PatchHdr h{};
+          h.cell0 = uint32_t(T.cells.size());
+          h.node0 = uint32_t(T.nodes.size());
+          h.ncells = uint16_t(n);
+          T.cells.insert(T.cells.end(), cells.begin() + c, cells.begin() + c + n);
+          table.clear();
+          for (size_t s = 0; s < n; ++s)
+            for (int j = 0; j < k; ++j) {
+              const uint32_t node = V.cell_nodes[size_t(cells[c + s]) * k + j];
+              if (table.insert(node)) T.nodes.push_back(node);
+            }
+          std::sort(T.nodes.begin() + h.node0, T.nodes.end());
+          h.nnodes = uint16_t(T.nodes.size() - h.node0);
+          h.nverts = uint16_t(std::lower_bound(T.nodes.begin() + h.node0, T.nodes.end(), uint32_t(m.nv)) -
+                              (T.nodes.begin() + h.node0));
+          T.max_nodes = std::max(T.max_nodes, int(h.nnodes));
+          T.max_verts = std::max(T.max_verts, int(h.nverts));
+          T.hdr.push_back(h);
+        }
+      }
+    }
+  }, 1);
+  std::vector<size_t> h0(nparts + 1, 0), c0(nparts + 1, 0), n0(nparts + 1, 0), k0(nparts + 1, 0);
+  for (int64_t i = 0; i < nparts; ++i) {
+    h0[i + 1] = h0[i] + parts[i].hdr.size();
+    c0[i + 1] = c0[i] + parts[i].cells.size();
+    n0[i + 1] = n0[i] + parts[i].nodes.size();
+    for (const PatchHdr& h : parts[i].hdr) B->stride = std::max<int>(B->stride, h.ncells);
+    B->max_nodes = std::max(B->max_nodes, parts[i].max_nodes);
+    B->max_verts = std::max(B->max_verts, parts[i].max_verts);
+  }
+  B->stride |= 1;
+  B->npatches = int64_t(h0[nparts]);
+  // how many patches hold each node; the shared ones' partial slots, filled in
+  // patch order
+  std::vector<uint32_t> slot(size_t(V.nnodes), 0);
+  for (const Part& T : parts)
+    for (uint32_t n : T.nodes) slot[n]++;
+  B->shared_ptr.push_back(0);
+  uint64_t acc = 0;
+  for (int64_t n = 0; n < V.nnodes; ++n) {
+    const uint32_t c = slot[n];
+    slot[n] = c > 1 ? uint32_t(acc) | kPatchPartial : 0u;
+    if (c != 1) {  // (c = 0, a vertex of no cell: an empty sum)
+      acc += c;
+      if (acc >= kPatchPartial) fail(DB2_ERR_UNSUPPORTED, "too many partial sums");
+      B->shared.push_back(uint32_t(n));
+      B->shared_ptr.push_back(uint32_t(acc));
+    }
+  }
+  B->nshared = int64_t(B->shared.size());
+  B->npartial = int64_t(acc);
+  std::vector<uint32_t> dest(n0[nparts]);
+  for (int64_t i = 0; i < nparts; ++i)
+    for (size_t s = 0; s < parts[i].nodes.size(); ++s) {
+      const uint32_t n = parts[i].nodes[s];
+      dest[n0[i] + s] = slot[n] & kPatchPartial ? slot[n]++ : n;
+    }
+  // pass 2: connectivity and jobs
+  parallel_for(nparts, [&](int64_t b, int64_t e) {
+    std::vector<uint32_t> ptr, order;
+    std::vector<uint16_t> list, codes;
+    std::vector<PatchGroup> groups;
+    std::vector<uint32_t> to, fill;
+    NodeTable table(size_t(max_cells) * k);
+    for (int64_t i = b; i < e; ++i) {
+      Part& T = parts[i];
+      T.conn.assign(T.cells.size() * kc, 0);
+      for (PatchHdr& h : T.hdr) {
+        const uint32_t* nodes = T.nodes.data() + h.node0;
+        uint16_t* conn = T.conn.data() + size_t(h.cell0) * kc;
+        ptr.assign(size_t(h.nnodes) + 1, 0);
+        table.clear();
+        for (int n = 0; n < h.nnodes; ++n) {
+          table.insert(nodes[n]);
+          table.val[table.find(nodes[n])] = uint32_t(n);
+        }
+        for (int c = 0; c < h.ncells; ++c) {
+          const uint32_t* cn = &V.cell_nodes[size_t(T.cells[h.cell0 + c]) * k];
+          for (int j = 0; j < k; ++j) {
+            const uint16_t ln = uint16_t(table.val[table.find(cn[j])]);
+            conn[size_t(c) * kc + j] = uint16_t(8 * ln);
+            ptr[ln + 1]++;
+          }
+        }
+        for (int n = 0; n < h.nnodes; ++n) ptr[n + 1] += ptr[n];
+        list.resize(ptr[h.nnodes]);
+        {
+          fill.assign(ptr.begin(), ptr.end() - 1);
+          for (int c = 0; c < h.ncells; ++c)
+            for (int j = 0; j < k; ++j) list[fill[conn[size_t(c) * kc + j] / 8]++] = uint16_t(8 * (j * B->stride + c));
+        }
+        // longest sums first, so that a group's lanes finish together
+        order.resize(h.nnodes);
+        std::iota(order.begin(), order.end(), 0u);
+        std::stable_sort(order.begin(), order.end(),
+                         [&](uint32_t a, uint32_t c) { return ptr[a + 1] - ptr[a] > ptr[c + 1] - ptr[c]; });
+        groups.clear();
+        codes.clear();
+        to.clear();
+        const uint16_t zero = uint16_t(8 * k * B->stride);
+        for (int g = 0; g < h.nnodes; g += 32) {
+          const int live = std::min(32, int(h.nnodes) - g);
+          const uint32_t width = ptr[order[g] + 1] - ptr[order[g]];
+          const size_t at = codes.size();
+          groups.push_back(PatchGroup{uint32_t(at), uint16_t(width), uint16_t(live)});
+          codes.resize(at + size_t(width) * 32, zero);
+          for (int l = 0; l < 32; ++l) {
+            to.push_back(l < live ? dest[n0[i] + h.node0 + order[g + l]] : 0u);
+            if (l < live)
+              for (uint32_t t = ptr[order[g + l]], q = 0; t < ptr[order[g + l] + 1]; ++t, ++q) codes[at + 32 * q + l] = list[t];
+          }
+        }
+        h.ngroups = uint16_t(groups.size());
+        h.chunk0 = uint32_t(T.chunks.size() / 16);
+        auto put = [&](const void* src, size_t bytes) {
+          const size_t a = T.chunks.size();
+          T.chunks.resize(a + PatchPlan::pad16(uint32_t(bytes)), 0);
+          if (bytes) std::memcpy(&T.chunks[a], src, bytes);
+        };
+        put(to.data(), to.size() * 4);
+        put(groups.data(), groups.size() * sizeof(PatchGroup));
+        put(codes.data(), codes.size() * 2);
+        h.chunks = uint32_t(T.chunks.size() / 16) - h.chunk0;
+        T.max_chunks = std::max<int>(T.max_chunks, int(h.chunks));
+      }
+    }
+  }, 1);
+  for (int64_t i = 0; i < nparts; ++i) {
+    k0[i + 1] = k0[i] + parts[i].chunks.size();
+    B->max_chunks = std::max(B->max_chunks, parts[i].max_chunks);
+  }
+  if (n0[nparts] >= (size_t(1) << 32) || k0[nparts] / 16 >= (size_t(1) << 32))
+    fail(DB2_ERR_UNSUPPORTED, "cell patches too large");
+  B->hdr.resize(h0[nparts]);
+  B->nodes.resize(n0[nparts]);
+  B->conn.resize(c0[nparts] * kc);
+  B->chunks.resize(k0[nparts]);
+  parallel_for(nparts, [&](int64_t b, int64_t e) {
+    for (int64_t i = b; i < e; ++i) {
+      Part& T = parts[i];
+      for (auto& h : T.hdr) {
+        h.cell0 += uint32_t(c0[i]);
+        h.node0 += uint32_t(n0[i]);
+        h.chunk0 += uint32_t(k0[i] / 16);
+      }
+      std::copy(T.hdr.begin(), T.hdr.end(), B->hdr.begin() + h0[i]);
+      std::copy(T.conn.begin(), T.conn.end(), B->conn.begin() + c0[i] * kc);
+      std::copy(T.nodes.begin(), T.nodes.end(), B->nodes.begin() + n0[i]);
+      if (!T.chunks.empty()) std::memcpy(B->chunks.data() + k0[i], T.chunks.data(), T.chunks.size());
+      T = Part();
+    }
+  }, 1);
+  return B;
+}
+
+// Cells of a patch: as many as let five 128-thread CTAs (four for elasticity)
+// share an SM.  Measured on B200 (ms per action): P2 tets n=96 0.246 with 330
+// cells (five CTAs) against 0.284 with 384 (four), 0.40 with 256; vector P2
+// elasticity n=48 0.089 with 200; P1 tets n=80 0.062 with 512, 0.066 with 768.
+// Small meshes are cut into about 600 patches (four for each of 148 SMs), down
+// to 64 cells: one patch's latency is the action's.
+const PatchPlan& patch_plan(const Pattern& P) {
+  if (!P.patches) {
+    const int full = P.V->degree == 1 ? 512 : P.bs > 1 ? 200 : 330;
+    auto B = make_patches(P, int(std::min<int64_t>(full, std::max<int64_t>(64, P.V->mesh->nc / 592))));
+    PlanUpload U;
+    auto up = [&](DeviceBuffer& d, auto& v) {
+      if (!v.empty()) U.put(d, v.data(), v.size() * sizeof(v[0]));
+      std::remove_reference_t<decltype(v)>().swap(v);
+    };
+    up(B->d_hdr, B->hdr);
+    up(B->d_conn, B->conn);
+    up(B->d_nodes, B->nodes);
+    up(B->d_chunks, B->chunks);
+    up(B->d_shared, B->shared);
+    up(B->d_shared_ptr, B->shared_ptr);
+    B->d_partial.alloc(size_t(B->npartial) * P.bs * sizeof(double));
+    P.patches = std::move(B);
+  }
+  return *P.patches;
+}
+
+}  // namespace db2
