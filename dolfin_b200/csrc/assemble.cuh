@@ -413,14 +413,20 @@ __device__ __forceinline__ void ld_rec4(const double* ptr, double& a, double& b,
                : "l"(ptr));
 }
 
-// Coordinates, kappa and f of one vertex (f from the vertex record in 2D,
-// from the P1 array in 3D).
-template <int D, bool FP1>
+// Coordinates, kappa and f of one vertex: kappa from its record (f too in 2D,
+// from the P1 array in 3D), or both from their arrays (DIRECT, for calls that
+// do not pack them into the records first).
+template <int D, bool FP1, bool DIRECT = false>
 __device__ __forceinline__ void load_vertex(const AsmParams& p, uint32_t v, double (&x)[D],
                                             double& kap, double& f) {
   double r0, r1, r2, r3;
   ld_rec4(p.xw + 4 * size_t(v), r0, r1, r2, r3);
-  if constexpr (D == 3) {
+  if constexpr (DIRECT) {
+    x[0] = r0; x[1] = r1;
+    if constexpr (D == 3) x[2] = r2;
+    kap = p.kappa ? __ldg(p.kappa + v) : 0.0;
+    f = FP1 ? __ldg(p.f + v) : 0.0;
+  } else if constexpr (D == 3) {
     x[0] = r0; x[1] = r1; x[2] = r2;
     kap = r3;
     f = FP1 ? __ldg(p.f + v) : 0.0;
@@ -470,23 +476,23 @@ __device__ __forceinline__ RowFix<D> load_row_fix(const AsmParams& p, uint32_t n
 }
 
 // Same with the kind of row known at compile time (NFIX fixed vertices).
-template <int D, int P, bool FP1, int NFIX>
+template <int D, int P, bool FP1, int NFIX, bool DIRECT>
 __device__ __forceinline__ RowFix<D> load_row_fix_n(const AsmParams& p, uint32_t node) {
   RowFix<D> r;
   r.nfix = NFIX;
   if constexpr (NFIX == 1) {
     r.base = node;
-    load_vertex<D, FP1>(p, node, r.x[0], r.kap[0], r.f[0]);
+    load_vertex<D, FP1, DIRECT>(p, node, r.x[0], r.kap[0], r.f[0]);
   } else {
     const uint2 e = __ldg(reinterpret_cast<const uint2*>(p.edge_v) + (node - p.nverts));
     r.base = e.x;
-    load_vertex<D, FP1>(p, e.x, r.x[0], r.kap[0], r.f[0]);
-    load_vertex<D, FP1>(p, e.y, r.x[1], r.kap[1], r.f[1]);
+    load_vertex<D, FP1, DIRECT>(p, e.x, r.x[0], r.kap[0], r.f[0]);
+    load_vertex<D, FP1, DIRECT>(p, e.y, r.x[1], r.kap[1], r.f[1]);
   }
   return r;
 }
 
-template <int D, int P, bool FP1, int NFIX, bool ESC>
+template <int D, int P, bool FP1, int NFIX, bool ESC, bool DIRECT>
 __device__ __forceinline__ void record_cell_n(const AsmParams& p, const RowFix<D>& F,
                                               const Rec<D, P>& r, uint32_t inc_index,
                                               double (&x)[D + 1][D],
@@ -503,7 +509,7 @@ __device__ __forceinline__ void record_cell_n(const AsmParams& p, const RowFix<D
       fv[a] = F.f[a];
     } else {
       const uint32_t v = esc ? pv[a] : uint32_t(int32_t(F.base) + r.delta(a - NFIX));
-      load_vertex<D, FP1>(p, v, x[a], kap[a], fv[a]);
+      load_vertex<D, FP1, DIRECT>(p, v, x[a], kap[a], fv[a]);
     }
   }
 }
@@ -525,7 +531,7 @@ __device__ __forceinline__ RowFixId load_row_fix_id(const AsmParams& p, uint32_t
   }
   return r;
 }
-template <int D, int P, bool FP1, int NFIX, bool ESC>
+template <int D, int P, bool FP1, int NFIX, bool ESC, bool DIRECT>
 __device__ __forceinline__ void record_cell_id(const AsmParams& p, const RowFixId& F,
                                                const Rec<D, P>& r, uint32_t inc_index,
                                                double (&x)[D + 1][D],
@@ -538,7 +544,7 @@ __device__ __forceinline__ void record_cell_id(const AsmParams& p, const RowFixI
     const uint32_t v = a < NFIX ? F.v[a]
                        : esc    ? pv[a]
                                 : uint32_t(int32_t(F.v[0]) + r.delta(a - NFIX));
-    load_vertex<D, FP1>(p, v, x[a], kap[a], fv[a]);
+    load_vertex<D, FP1, DIRECT>(p, v, x[a], kap[a], fv[a]);
   }
 }
 
@@ -668,7 +674,11 @@ __device__ __forceinline__ double load_row(const AsmParams& p, const Geometry<D>
 // Variant flags of the tile kernel (separate instantiations, so that the
 // common case pays for neither): records with escaped vertex offsets, and
 // Dirichlet data (without it the row walk carries no boundary-condition state).
-enum { VAR_ESC = 1, VAR_BC = 2 };
+// VAR_LAT: small problems, whose rows do not fill the SMs and whose time is one
+// row walk's latency -- the next incidence's vertices are loaded one incidence
+// ahead (registers to spare there), and kappa and f come from their arrays, so
+// that no packing launch precedes the tiles.
+enum { VAR_ESC = 1, VAR_BC = 2, VAR_LAT = 4 };
 
 template <int D, int P, int FORM, bool KP1, int LOADM, typename CT, int NFIX, int VAR>
 __device__ __forceinline__ void row_unit(const AsmParams& p, const Tile& t, CT* acc,
@@ -677,7 +687,7 @@ __device__ __forceinline__ void row_unit(const AsmParams& p, const Tile& t, CT* 
   constexpr int BS = FORM == FORM_ELAS ? D : 1;
   constexpr bool FP1 = LOADM == LOAD_P1 || LOADM == LOAD_KP1;
   constexpr bool vertex = NFIX == 1;
-  constexpr bool ESC = (VAR & VAR_ESC) != 0;
+  constexpr bool ESC = (VAR & VAR_ESC) != 0, LAT = (VAR & VAR_LAT) != 0;
   const bool bc = (VAR & VAR_BC) != 0 && p.bc_flags != nullptr;
   const uint32_t node = t.n0 + u / BS;
   const int e = u % BS;
@@ -701,11 +711,11 @@ __device__ __forceinline__ void row_unit(const AsmParams& p, const Tile& t, CT* 
   // hits); the Poisson rows keep them in registers (measured on B200:
   // reloading costs 10 % on P2 Poisson; elasticity with first-touch stores at
   // 96 registers: 1.20 ms reloading against 1.32 keeping them).
-  constexpr bool RELOAD = FORM == FORM_ELAS;
+  constexpr bool RELOAD = FORM == FORM_ELAS && !LAT;
   using Fix = typename std::conditional<RELOAD, RowFixId, RowFix<D>>::type;
   Fix F;
   if constexpr (RELOAD) F = load_row_fix_id<D, P, NFIX>(p, node);
-  else F = load_row_fix_n<D, P, FP1, NFIX>(p, node);
+  else F = load_row_fix_n<D, P, FP1, NFIX, LAT>(p, node);
   // The unit owns acc[my, my + L) alone (the units' segments partition the
   // tile's), so it clears its own segment: no block barrier before the row
   // walk, whose first loads are already in flight.
@@ -736,12 +746,36 @@ __device__ __forceinline__ void row_unit(const AsmParams& p, const Tile& t, CT* 
   // copy, so it is issued beside the row's other loads, not after rec_goff.
   Rec<D, P> rn{};
   if (cnt > 0) rn = load_rec_from<D, P>(p.rec_first, node);
+  auto cell_of = [&](const Rec<D, P>& r, uint32_t m, double (&x)[D + 1][D], double (&kap)[D + 1],
+                     double (&fv)[D + 1]) {
+    if constexpr (RELOAD) record_cell_id<D, P, FP1, NFIX, ESC, LAT>(p, F, r, i0 + m, x, kap, fv);
+    else record_cell_n<D, P, FP1, NFIX, ESC, LAT>(p, F, r, i0 + m, x, kap, fv);
+  };
+  // VAR_LAT: the record after the next, and the next cell
+  Rec<D, P> rnn{};
+  double xn[D + 1][D], kn[D + 1], fn[D + 1];
+  if constexpr (LAT) {
+    if (cnt > 0) cell_of(rn, 0, xn, kn, fn);
+    if (cnt > 1) rnn = load_rec<D, P>(p, rbase + 32u);
+  }
   for (uint32_t m = 0; m < cnt; ++m) {
     const Rec<D, P> r = rn;
-    if (m + 1 < cnt) rn = load_rec<D, P>(p, rbase + 32u * (m + 1));
     double x[D + 1][D], kap[D + 1], fv[D + 1];
-    if constexpr (RELOAD) record_cell_id<D, P, FP1, NFIX, ESC>(p, F, r, i0 + m, x, kap, fv);
-    else record_cell_n<D, P, FP1, NFIX, ESC>(p, F, r, i0 + m, x, kap, fv);
+    if constexpr (LAT) {
+#pragma unroll
+      for (int a = 0; a <= D; ++a) {
+#pragma unroll
+        for (int q = 0; q < D; ++q) x[a][q] = xn[a][q];
+        kap[a] = kn[a];
+        fv[a] = fn[a];
+      }
+      rn = rnn;
+      if (m + 1 < cnt) cell_of(rn, m + 1, xn, kn, fn);
+      if (m + 2 < cnt) rnn = load_rec<D, P>(p, rbase + 32u * (m + 2));
+    } else {
+      if (m + 1 < cnt) rn = load_rec<D, P>(p, rbase + 32u * (m + 1));
+      cell_of(r, m, x, kap, fv);
+    }
     Geometry<D> G;
     geometry(x, G);
     CT out[E::K];
@@ -916,9 +950,10 @@ __device__ __forceinline__ void tile_body(const AsmParams& p, const Tile t, doub
 #ifndef DB2_TILE_MAXNREG_ELAS
 #define DB2_TILE_MAXNREG_ELAS 96
 #endif
-template <int P, int FORM, typename CT>
+template <int P, int FORM, typename CT, int VAR>
 constexpr int tile_maxnreg() {
-  return sizeof(CT) == 4       ? DB2_TILE_MAXNREG_F32
+  return (VAR & VAR_LAT) ? 255
+         : sizeof(CT) == 4       ? DB2_TILE_MAXNREG_F32
          : FORM == FORM_ELAS ? DB2_TILE_MAXNREG_ELAS
          : P == 1            ? DB2_TILE_MAXNREG_P1
                              : DB2_TILE_MAXNREG_P2;
@@ -926,9 +961,12 @@ constexpr int tile_maxnreg() {
 // VAR: VAR_ESC when the pattern has records whose vertex offsets did not fit
 // 16 bits, VAR_BC when the call has Dirichlet data.
 template <int D, int P, int FORM, bool KP1, int LOADM, typename CT, int VAR>
-__global__ void __maxnreg__((tile_maxnreg<P, FORM, CT>())) k_assemble(const AsmParams p) {
+__global__ void __maxnreg__((tile_maxnreg<P, FORM, CT, VAR>())) k_assemble(const AsmParams p) {
   extern __shared__ __align__(16) double acc[];
-  tile_body<D, P, FORM, KP1, LOADM, CT, VAR>(p, p.tiles[blockIdx.x], acc);
+  // one launch for all classes (VAR_LAT): the last class's tiles, vertex rows with
+  // the longest walks, start first
+  tile_body<D, P, FORM, KP1, LOADM, CT, VAR>(
+      p, p.tiles[(VAR & VAR_LAT) ? gridDim.x - 1 - blockIdx.x : blockIdx.x], acc);
 }
 
 }  // namespace dev

@@ -134,6 +134,25 @@ static int load_mode(const FormArgs* L, int bs, dev::AsmParams& p) {
   }
 }
 
+// Incidences (row, cell, trial and test component) up to which a pattern is
+// assembled for latency: VAR_LAT, one launch instead of a packing launch and
+// one per tile class with its fork and join.  Below the line the call's time is
+// launches and one row walk; above it the row walks' throughput, where the
+// extra registers cost residency.  Measured on B200 (us a call, tile classes ->
+// one launch): P2 tets n=10 36 -> 14, n=22 (0.64 M incidences) 37 -> 19, n=26
+// (1.05 M) 40 -> 36, n=36 (2.8 M) 78 -> 79; P1 tets n=34 (0.94 M) 23 -> 18, n=38
+// (1.3 M) 21 -> 21, n=44 (2.0 M) 31 -> 38; vector P2 elasticity n=12 (0.93 M)
+// 35 -> 25, n=14 (1.5 M) 35 -> 35; P2 triangles n=200 (0.48 M) 21 -> 14, n=300
+// (1.08 M) 29 -> 30.  FP32 rows of P2 tets spill at their register cap in the
+// tile classes: n=34 (2.4 M) 75 -> 60, n=37 (3.0 M) 86 -> 76, elasticity n=14
+// 49 -> 38, n=18 (3.1 M) 70 -> 69.  By the pattern's size, not the row range's,
+// so that a range's rows equal the whole assembly's bit for bit.
+static bool latency_bound(const Pattern& P, bool fp32) {
+  const int64_t incidences = int64_t(P.inc.size()) * P.bs * P.bs;
+  const int64_t line = P.V->mesh->tdim == 2 ? 1000000 : fp32 && P.V->degree == 2 ? 3000000 : 1400000;
+  return incidences <= line && P.rec_escapes == 0;
+}
+
 void launch_assemble(const Pattern& P, const FormArgs* a, const FormArgs* L, int precision,
                      double* vals, double* b, bool add_values, const uint8_t* bc_flags,
                      const double* bc_vals, void* stream) {
@@ -187,12 +206,14 @@ void launch_assemble(const Pattern& P, const FormArgs* a, const FormArgs* L, int
   cfg.stream = static_cast<cudaStream_t>(stream);
   cfg.escapes = P.rec_escapes > 0;
   const bool fp32 = precision == DB2_FP32_CONTRACT;
+  cfg.latency = latency_bound(P, fp32);
   if (precision != DB2_FP64 && precision != DB2_FP32_CONTRACT) fail(DB2_ERR_ARGUMENT, "unknown precision %d", precision);
   bool ok = false;
   if (a->f.kind == DB2_FORM_DIFFUSION) {
     if (P.bs != 1) fail(DB2_ERR_UNSUPPORTED, "diffusion form on a vector space");
     const bool kp1 = matrix_coeff(*a, p);
-    pack_vertex_records(P, kp1 ? p.kappa : nullptr,
+    if (!cfg.latency)
+      pack_vertex_records(P, kp1 ? p.kappa : nullptr,
                         (loadm == dev::LOAD_P1 || loadm == dev::LOAD_KP1) ? p.f : nullptr, stream);
     ok = D == 3 ? dev::dispatch_tet_diff(V.degree, p, cfg, kp1, loadm, fp32)
                 : dev::dispatch_tri_diff(V.degree, p, cfg, kp1, loadm, fp32);

@@ -14,6 +14,7 @@ struct LaunchCfg {
   int threads;
   cudaStream_t stream;
   bool escapes = false;  // the pattern has records with escaped vertex offsets
+  bool latency = false;  // a small problem: VAR_LAT, and one launch for all tile classes
 };
 
 // Let `kern` use all the dynamic shared memory the current device allows a
@@ -71,14 +72,30 @@ inline SideStreams& side_streams() {
 // alone below the SM's residency limits.
 template <int D, int P, int FORM, bool KP1, int LOADM, typename CT>
 void run_assemble(const AsmParams& p, const LaunchCfg& cfg) {
-  const int var = (cfg.escapes ? VAR_ESC : 0) | (p.bc_flags ? VAR_BC : 0);
-  auto kern = var == 0         ? k_assemble<D, P, FORM, KP1, LOADM, CT, 0>
+  const int var = (cfg.escapes ? VAR_ESC : 0) | (p.bc_flags ? VAR_BC : 0) | (cfg.latency ? VAR_LAT : 0);
+  auto kern = var == VAR_LAT              ? k_assemble<D, P, FORM, KP1, LOADM, CT, VAR_LAT>
+              : var == (VAR_LAT | VAR_BC) ? k_assemble<D, P, FORM, KP1, LOADM, CT, VAR_LAT | VAR_BC>
+              : var == 0         ? k_assemble<D, P, FORM, KP1, LOADM, CT, 0>
               : var == VAR_ESC ? k_assemble<D, P, FORM, KP1, LOADM, CT, VAR_ESC>
               : var == VAR_BC  ? k_assemble<D, P, FORM, KP1, LOADM, CT, VAR_BC>
                                : k_assemble<D, P, FORM, KP1, LOADM, CT, VAR_ESC | VAR_BC>;
-  static unsigned long long configured[4] = {0, 0, 0, 0};
+  static unsigned long long configured[8] = {};
   allow_dynamic_smem(kern, configured[var]);
   const auto& cb = *cfg.class_begin;
+  if (cfg.latency) {
+    // every tile at once, with the largest class's shared memory
+    const int n = cb.back() - cb.front();
+    if (n > 0) {
+      AsmParams q = p;
+      q.tiles = p.tiles + cb.front();
+      const size_t smem = size_t(cfg.class_smem->back()) * sizeof(CT) / sizeof(double) +
+                          size_t(cfg.threads) * sizeof(double) + 16;
+      kern<<<n, cfg.threads, smem, cfg.stream>>>(q);
+      count_launch();
+      check_cuda("assemble launch");
+    }
+    return;
+  }
   const int ncls = int(cb.size()) - 1;
   const bool fork = DB2_CLASS_STREAMS && ncls > 1 && ncls <= SideStreams::kMax;
   SideStreams* S = fork ? &side_streams() : nullptr;
