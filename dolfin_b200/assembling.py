@@ -182,6 +182,14 @@ class SystemAssembler:
         self.prec = _PREC[precision]
         self.keep_diagonal = False
 
+    @classmethod
+    def _of(cls, ra, rL, precision):
+        """The assembler of recognised cell forms (kappa grad.grad and a load)."""
+        S = cls.__new__(cls)
+        S.ra, S.rL, S.ra_ds, S.rL_ds, S.bcs = ra, rL, None, None, []
+        S.prec, S.keep_diagonal = _PREC[precision], False
+        return S
+
     def assemble(self, A=None, b=None):
         V = self.ra.V
         if A is None and b is None:
@@ -264,12 +272,16 @@ def assemble_action(a, x, y=None, precision="fp64"):
 
 
 def _bc_arrays(V, bcs):
+    """Dirichlet flags and values over the dofs, from the conditions' dofs and
+    values kept on the device (copying them from the host at every call cost
+    about 100 us and a synchronisation)."""
     import torch
     flags = torch.zeros(V.dim(), dtype=torch.uint8, device="cuda")
     vals = torch.zeros(V.dim(), dtype=torch.float64, device="cuda")
     for bc in bcs:
-        dofs, values = bc.dofs_and_values()
-        d = torch.as_tensor(dofs, dtype=torch.int64, device="cuda")
-        flags[d] = 1
-        vals[d] = torch.as_tensor(values, dtype=torch.float64, device="cuda")
+        dofs, values = bc.device_dofs_and_values()
+        for t in (dofs, values):  # they may have been made on another stream
+            t.record_stream(torch.cuda.current_stream())
+        flags.index_fill_(0, dofs, 1)
+        vals.index_copy_(0, dofs, values)
     return flags, vals

@@ -41,6 +41,7 @@ class DirichletBC:
         self.value = value
         self.where = where
         self._cache = None
+        self._device = {}
 
     def function_space(self):
         return self.V
@@ -106,6 +107,16 @@ class DirichletBC:
         values = np.concatenate([vals[:, c] for c in range(vs)])
         self._cache = (dofs, values)
         return self._cache
+
+    def device_dofs_and_values(self):
+        """dofs_and_values() as tensors on the current CUDA device."""
+        import torch
+        dev = torch.cuda.current_device()
+        if dev not in self._device:
+            dofs, values = self.dofs_and_values()
+            self._device[dev] = (torch.as_tensor(dofs, dtype=torch.int64, device="cuda"),
+                                 torch.as_tensor(values, dtype=torch.float64, device="cuda"))
+        return self._device[dev]
 
     def _values(self, pts, vs, n):
         from .function import Constant

@@ -364,6 +364,7 @@ class Recognised:
         # a load c*f1*f2*v*dx: the two P1 Functions (which one is kappa is
         # decided by the bilinear form it is assembled with)
         self.pair = pair
+        self._c = None
 
     def with_kappa(self, kappa):
         """The load c*kappa*f*v*dx of a two-Function load, kappa being the
@@ -376,8 +377,11 @@ class Recognised:
         return Recognised(self.kind, self.V, _capi.COEFF_P1_KAPPA, f, self.constant)
 
     def c_form(self):
-        from . import _capi
-        return _capi.make_form(self.kind, self.coeff, self.constant, self.mu, self.lmbda)
+        """The C form (made once: a recognised form does not change)."""
+        if self._c is None:
+            from . import _capi
+            self._c = _capi.make_form(self.kind, self.coeff, self.constant, self.mu, self.lmbda)
+        return self._c
 
     def __repr__(self):
         return (f"Recognised(kind={self.kind}, coeff={self.coeff}, constant={self.constant}, "
