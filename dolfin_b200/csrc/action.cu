@@ -3,10 +3,8 @@
 // coefficient.
 #include <cuda_runtime.h>
 
-#include <utility>
-
 #include "launch.cuh"
-#include "quad.cuh"
+#include "adjoint.cuh"
 #include "action_tc.cuh"
 
 #include <algorithm>
@@ -28,77 +26,30 @@ __global__ void __launch_bounds__(256) k_apply_gather(const uint32_t* __restrict
   y[node] = acc;
 }
 
-// Adjoint, step 1, the part of local node LI of the cell (a compile-time
-// relabelling, so the permuted geometry tensor is register renaming):
-// acc[a] += sum_j gA_(LI,j) dA^K_(LI,j)/dkappa_a + gb_LI db^K_LI/dkappa_a.
-// Wn[a][b] = n_a . n_b in the cell's own vertex order; under the relabelling
-// n'_a = +-n_perm[a], so W'_ab = Wn[perm[a]][perm[b]] (|det J| unchanged).
-template <int D, int P, bool LOADK, typename CT, int LI>
-__device__ __forceinline__ void vjp_node(const AsmParams& p, int64_t cell,
-                                         const double (&Wn)[D + 1][D + 1], double s, double vol,
-                                         const double (&fv)[D + 1], const double* __restrict__ gA,
-                                         const double* __restrict__ gb, double (&acc)[D + 1]) {
-  using E = El<D, P>;
-  using R = Rows<D, P, CT>;
-  constexpr int NB = D + 1;
-  constexpr uint32_t code = perm_code(D, LI);
-  constexpr bool vertex = LI <= D;
-  const uint32_t ii = __ldg(p.cell_inc + size_t(cell) * E::K + LI);
-  const uint32_t node = __ldg(p.cell_nodes + size_t(cell) * E::K + LI);
-  const double* grow = gA + __ldg(p.node_rowptr + node);
-  // gA at the row's slots, in the relabelled local order
-  double g[E::K];
-  const Rec<D, P> rr = load_rec<D, P>(p, rec_index<D, P>(p, node, ii - __ldg(p.inc_ptr + node)));
+// gA at the columns of a cell's row by its incidence record, and gb.
+template <int D, int P, bool LOADK>
+struct RecordRow {
+  const AsmParams& p;
+  int64_t cell;
+  const uint32_t (&v)[D + 1];          // the cell's vertices
+  const uint32_t (&inc)[El<D, P>::K];  // and incidences
+  const double* gA;
+  const double* gb;
+  template <int LI>
+  __device__ __forceinline__ void get(double (&g)[El<D, P>::K], double& gbi) const {
+    constexpr int K = El<D, P>::K;
+    const uint32_t ii = inc[LI];
+    // vertex nodes are numbered as the vertices (natural numbering)
+    uint32_t node;
+    if constexpr (LI <= D) node = v[LI];
+    else node = __ldg(p.cell_nodes + size_t(cell) * K + LI);
+    const double* grow = gA + __ldg(p.node_rowptr + node);
+    const Rec<D, P> rr = load_rec<D, P>(p, rec_index<D, P>(p, node, ii - __ldg(p.inc_ptr + node)));
 #pragma unroll
-  for (int j = 0; j < E::K; ++j) g[j] = __ldg(grow + rr.slot(j));
-  auto pm = [](int a) { return int((code >> (2 * a)) & 3u); };
-  CT W0[1][NB];
-  CT W1[2][NB];
-  // W times the generated rows' scale (see element_rows.h)
-  const double sv = s * (p.kscale * R::sv_kp1);
-#pragma unroll
-  for (int b = 0; b < NB; ++b) W0[0][b] = CT(Wn[pm(0)][pm(b)] * sv);
-  if constexpr (P == 2) {
-    const double se = s * (p.kscale * R::se_kp1);
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int b = 0; b < NB; ++b) W1[a][b] = CT(Wn[pm(a)][pm(b)] * se);
+    for (int j = 0; j < K; ++j) g[j] = __ldg(grow + rr.slot(j));
+    if constexpr (LOADK) gbi = __ldg(gb + node);
   }
-  CT lk[NB];
-  if constexpr (LOADK) {
-    CT fc[NB];
-#pragma unroll
-    for (int a = 0; a < NB; ++a) fc[a] = CT(fv[pm(a)]);
-    if constexpr (P == 2 && !vertex) R::e_kfp1(fc, lk);
-    else R::v_kfp1(fc, lk);
-  }
-  const double gbi = LOADK ? __ldg(gb + node) : 0.0;
-#pragma unroll
-  for (int m = 0; m < NB; ++m) {
-    CT unit[NB];
-#pragma unroll
-    for (int a = 0; a < NB; ++a) unit[a] = CT(a == m ? 1 : 0);
-    CT d[E::K];
-    if constexpr (P == 1 || vertex) R::v_kp1(W0, unit, d);
-    else R::e_kp1(W1, unit, d);
-    double t = 0.0;
-#pragma unroll
-    for (int j = 0; j < E::K; ++j) t = fma(g[j], double(d[j]), t);
-    if constexpr (LOADK) t = fma(gbi, vol * double(lk[m]) * p.fc[0], t);
-    // relabelled vertex m is original local vertex perm[m]
-    acc[pm(m)] += t;
-  }
-}
-
-template <int D, int P, bool LOADK, typename CT, int... LI>
-__device__ __forceinline__ void vjp_nodes(const AsmParams& p, int64_t cell,
-                                          const double (&Wn)[D + 1][D + 1], double s, double vol,
-                                          const double (&fv)[D + 1], const double* gA,
-                                          const double* gb, double (&acc)[D + 1],
-                                          std::integer_sequence<int, LI...>) {
-  (vjp_node<D, P, LOADK, CT, LI>(p, cell, Wn, s, vol, fv, gA, gb, acc), ...);
-}
+};
 
 // Adjoint, step 1 (one thread per cell): t[cell][m] = sum_{i,j in cell}
 // gA_ij dA^K_ij/dkappa_m + sum_i gb_i db^K_i/dkappa_m for the P1 kappa
@@ -122,6 +73,27 @@ __global__ void __maxnreg__((vjp_maxnreg<P>())) k_vjp_cells(const AsmParams p, i
   if (cell >= ncells) return;
   uint32_t v[NB];
   load_verts<D>(p, uint32_t(cell), v);
+  // the cell's incidences, in the widest loads its row of the array allows
+  uint32_t inc[E::K];
+  {
+    const uint32_t* ci = p.cell_inc + size_t(cell) * E::K;
+    if constexpr (E::K % 4 == 0) {
+#pragma unroll
+      for (int j = 0; j < E::K; j += 4) {
+        const uint4 w = __ldg(reinterpret_cast<const uint4*>(ci + j));
+        inc[j] = w.x; inc[j + 1] = w.y; inc[j + 2] = w.z; inc[j + 3] = w.w;
+      }
+    } else if constexpr (E::K % 2 == 0) {
+#pragma unroll
+      for (int j = 0; j < E::K; j += 2) {
+        const uint2 w = __ldg(reinterpret_cast<const uint2*>(ci + j));
+        inc[j] = w.x; inc[j + 1] = w.y;
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < E::K; ++j) inc[j] = __ldg(ci + j);
+    }
+  }
   double x[NB][D], kap_unused[NB], f_unused[NB];
   load_vertex_data<D, false>(p, v, x, kap_unused, f_unused);
   double fv[NB];
@@ -137,11 +109,12 @@ __global__ void __maxnreg__((vjp_maxnreg<P>())) k_vjp_cells(const AsmParams p, i
   double acc[NB];
 #pragma unroll
   for (int a = 0; a < NB; ++a) acc[a] = 0.0;
-  vjp_nodes<D, P, LOADK, CT>(p, cell, Wn, G.s, G.vol, fv, gA, gb, acc,
-                             std::make_integer_sequence<int, E::K>{});
+  const RecordRow<D, P, LOADK> row{p, cell, v, inc, gA, gb};
+  vjp_nodes<D, P, LOADK, CT>(p, Wn, G.s, G.vol, fv, row, acc, std::make_integer_sequence<int, E::K>{});
   // in vertex-incidence order (vertex nodes come first in the node-contiguous
   // incidence array), so that step 2 reads each vertex's terms contiguously
-  for (int a = 0; a < NB; ++a) t[__ldg(p.cell_inc + size_t(cell) * E::K + a)] = acc[a];
+#pragma unroll
+  for (int a = 0; a < NB; ++a) t[inc[a]] = acc[a];
 }
 
 // Adjoint, step 2 (one thread per vertex): dkappa[v] = sum over cells around

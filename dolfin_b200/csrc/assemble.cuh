@@ -27,6 +27,7 @@
 #include <type_traits>
 
 #include "generated/element_rows.h"
+#include "kappa_rows.cuh"
 #include "internal.h"
 
 namespace db2 {
@@ -226,7 +227,8 @@ struct Rows;
     }                                                                                      \
     __device__ static void v_kp1(const CT (&W)[1][D_ + 1], const CT (&k)[D_ + 1],           \
                                  CT (&o)[K_]) {                                            \
-      gen::grad_grad_##NAME##_v_kp1<CT>(W, k, o);                                           \
+      if constexpr (P_ == 2 && sizeof(CT) == 8) p2_kappa_vertex_row(W, k, o);               \
+      else gen::grad_grad_##NAME##_v_kp1<CT>(W, k, o);                                      \
     }                                                                                      \
     __device__ static double v_f1() { return gen::load_##NAME##_v_f1<double>(); }           \
     __device__ static double v_fp1(const double (&f)[D_ + 1]) {                             \
@@ -242,7 +244,8 @@ struct Rows;
     gen::grad_grad_##NAME##_e_k1<CT>(W, o);                                                 \
   }                                                                                        \
   __device__ static void e_kp1(const CT (&W)[2][D_ + 1], const CT (&k)[D_ + 1], CT (&o)[K_]) { \
-    gen::grad_grad_##NAME##_e_kp1<CT>(W, k, o);                                             \
+    if constexpr (sizeof(CT) == 8) p2_kappa_edge_row(W, k, o);                              \
+    else gen::grad_grad_##NAME##_e_kp1<CT>(W, k, o);                                        \
   }                                                                                        \
   __device__ static double e_f1() { return gen::load_##NAME##_e_f1<double>(); }             \
   __device__ static double e_fp1(const double (&f)[D_ + 1]) {                               \

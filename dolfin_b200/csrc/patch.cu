@@ -14,43 +14,20 @@
 // 0.081 (its quadrature is unchanged, and issue-bound).
 #include <cuda_runtime.h>
 
-#include "launch.cuh"
+#include "patch.cuh"
 #include "quad.cuh"
 
 namespace db2 {
 namespace dev {
 
-struct PatchArgs {
-  const PatchHdr* hdr;
-  const uint16_t* conn;
-  const uint32_t* nodes;
-  const uint4* chunks;
+struct PatchArgs : PatchView {
   const double* xw;     // vertex records, coordinates first
   const double* kappa;  // P1 field or null
   double kscale, mu, lmbda;
   const double* x;
   double* y;
-  double* partial;
-  int64_t nnodes, npartial;
-  int stride;           // staged cells of a local node
-  int nx, nv;           // room for the patch's nodes and vertices
-  uint32_t ahead;       // patches in flight on the device
+  int64_t nnodes;
 };
-
-__device__ __forceinline__ PatchHdr patch_header(const PatchHdr* hdr, uint32_t i) {
-  const uint4* s = reinterpret_cast<const uint4*>(hdr + i);
-  const uint4 a = __ldg(s), b = __ldg(s + 1);
-  PatchHdr h;
-  h.cell0 = a.x;
-  h.node0 = a.y;
-  h.chunk0 = a.z;
-  h.chunks = a.w;
-  h.ncells = uint16_t(b.x & 0xffffu);
-  h.nnodes = uint16_t(b.x >> 16);
-  h.nverts = uint16_t(b.y & 0xffffu);
-  h.ngroups = uint16_t(b.y >> 16);
-  return h;
-}
 
 // Element action of P2 by exact moments, FP64.  With U_m the gradient of u at
 // vertex m (grad u is linear), F the flux and M_m = int lambda_m F:
@@ -307,19 +284,10 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
   const uint32_t later = blockIdx.x + q.ahead;
   PatchHdr hn{};
   if (later < gridDim.x) hn = patch_header(q.hdr, later);
-  {
-    const uint4* src = q.chunks + h.chunk0;
-    const uint32_t to = static_cast<uint32_t>(__cvta_generic_to_shared(jobs));
-    for (uint32_t i = threadIdx.x; i < h.chunks; i += T)
-      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(to + 16u * i), "l"(src + i) : "memory");
-  }
+  patch_jobs_copy(q, h, jobs);
   // the cells' local nodes are loaded one cell ahead
-  constexpr int KC = patch_conn(K) / 4;
-  const uint2* conn = reinterpret_cast<const uint2*>(q.conn) + size_t(h.cell0) * KC;
-  uint2 cn[KC];
-#pragma unroll
-  for (int i = 0; i < KC; ++i)
-    cn[i] = int(threadIdx.x) < h.ncells ? __ldg(conn + threadIdx.x * KC + i) : make_uint2(0u, 0u);
+  PatchCell<K> cn{};
+  if (int(threadIdx.x) < h.ncells) cn.load(q, h, threadIdx.x);
   for (int i = threadIdx.x; i < h.nnodes; i += T) {
     const uint32_t node = __ldg(q.nodes + h.node0 + i);
 #pragma unroll
@@ -333,27 +301,14 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
     }
   }
   if (threadIdx.x < BS) ys[threadIdx.x * plane + K * q.stride] = CT(0);
-  asm volatile("cp.async.wait_all;" ::: "memory");
+  patch_jobs_wait();
   __syncthreads();
-  if (later < gridDim.x) {
-    auto prefetch = [](const void* p, uint32_t bytes) {
-      const char* b = static_cast<const char*>(p);
-      for (uint32_t i = 128u * threadIdx.x; i < bytes; i += 128u * T)
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(b + i));
-    };
-    prefetch(q.nodes + hn.node0, hn.nnodes * 4u);
-    prefetch(reinterpret_cast<const uint2*>(q.conn) + size_t(hn.cell0) * KC, hn.ncells * KC * 8u);
-    prefetch(q.chunks + hn.chunk0, hn.chunks * 16u);
-  }
+  if (later < gridDim.x) patch_prefetch<K>(q, hn);
   for (int c = threadIdx.x; c < h.ncells; c += T) {
     double xv[NB][D], kap[NB], xc[BS][K], y[BS][K];
-    auto off = [&](int j) {  // 8 x local node j
-      const uint32_t w = (j & 2) ? cn[j >> 2].y : cn[j >> 2].x;
-      return (j & 1) ? w >> 16 : w & 0xffffu;
-    };
 #pragma unroll
     for (int a = 0; a < NB; ++a) {
-      const double2* v = reinterpret_cast<const double2*>(reinterpret_cast<const char*>(vs) + 4 * off(a));
+      const double2* v = reinterpret_cast<const double2*>(reinterpret_cast<const char*>(vs) + 4 * cn.off(a));
       const double2 lo = v[0], hi = v[1];
       xv[a][0] = lo.x;
       xv[a][1] = lo.y;
@@ -362,14 +317,11 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
     }
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      const char* xj = reinterpret_cast<const char*>(xs) + off(j);
+      const char* xj = reinterpret_cast<const char*>(xs) + cn.off(j);
 #pragma unroll
       for (int e = 0; e < BS; ++e) xc[e][j] = reinterpret_cast<const double*>(xj)[e * q.nx];
     }
-    if (c + T < h.ncells) {
-#pragma unroll
-      for (int i = 0; i < KC; ++i) cn[i] = __ldg(conn + (c + T) * KC + i);
-    }
+    if (c + T < h.ncells) cn.load(q, h, c + T);
     cell_action<D, P, FORM, KP1, CT>(q, xv, kap, xc, y);
 #pragma unroll
     for (int e = 0; e < BS; ++e)
@@ -377,14 +329,11 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
       for (int j = 0; j < K; ++j) ys[e * plane + j * q.stride + c] = CT(y[e][j]);
   }
   __syncthreads();
-  const uint32_t* dest = reinterpret_cast<const uint32_t*>(jobs);
-  const PatchGroup* groups = reinterpret_cast<const PatchGroup*>(jobs + 128u * h.ngroups);
-  const uint16_t* codes = reinterpret_cast<const uint16_t*>(
-      jobs + 128u * h.ngroups + PatchPlan::pad16(h.ngroups * uint32_t(sizeof(PatchGroup))));
+  const PatchJobs J = patch_jobs(h, jobs);
   const int lane = threadIdx.x & 31;
   for (int g = threadIdx.x >> 5; g < h.ngroups; g += T / 32) {
-    const PatchGroup gr = groups[g];
-    const uint16_t* code = codes + gr.code0 + lane;
+    const PatchGroup gr = J.groups[g];
+    const uint16_t* code = J.codes + gr.code0 + lane;
     double acc[BS];
 #pragma unroll
     for (int e = 0; e < BS; ++e) acc[e] = 0.0;
@@ -396,7 +345,7 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
       for (int e = 0; e < BS; ++e) acc[e] += double(v[e * plane]);
     }
     if (lane < gr.live) {
-      const uint32_t d = dest[32 * g + lane];
+      const uint32_t d = J.dest[32 * g + lane];
       double* out = d & kPatchPartial ? q.partial + (d & ~kPatchPartial) : q.y + d;
       const int64_t step = d & kPatchPartial ? q.npartial : q.nnodes;
 #pragma unroll
@@ -405,27 +354,8 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
   }
 }
 
-// Nodes shared between patches: their partial sums in patch order.
-template <int BS>
-__global__ void __launch_bounds__(256) k_patch_sum(const uint32_t* __restrict__ shared,
-                                                   const uint32_t* __restrict__ ptr, int64_t n,
-                                                   const double* __restrict__ partial, int64_t npartial,
-                                                   double* __restrict__ y, int64_t nnodes) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint32_t node = __ldg(shared + i), s0 = __ldg(ptr + i), s1 = __ldg(ptr + i + 1);
-  double acc[BS];
-#pragma unroll
-  for (int e = 0; e < BS; ++e) acc[e] = 0.0;
-  for (uint32_t s = s0; s < s1; ++s)
-#pragma unroll
-    for (int e = 0; e < BS; ++e) acc[e] += __ldg(partial + int64_t(e) * npartial + s);
-#pragma unroll
-  for (int e = 0; e < BS; ++e) y[int64_t(e) * nnodes + node] = acc[e];
-}
-
 template <int D, int P, int FORM, bool KP1, typename CT>
-void run_patch_apply(const PatchPlan& B, PatchArgs q, cudaStream_t s) {
+void run_patch_apply(const PatchPlan& B, const PatchArgs& q, cudaStream_t s) {
   constexpr int K = El<D, P>::K, BS = FORM == FORM_ELAS ? D : 1;
   if (B.npatches > 0) {
     auto kern = k_patch_apply<D, P, FORM, KP1, CT>;
@@ -433,10 +363,6 @@ void run_patch_apply(const PatchPlan& B, PatchArgs q, cudaStream_t s) {
     allow_dynamic_smem(kern, configured);
     const size_t smem = PatchPlan::pad16(uint32_t((4 * q.nv + BS * q.nx) * 8 + BS * (K * q.stride + 1) * int(sizeof(CT)))) +
                         size_t(B.max_chunks) * 16;
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    q.ahead = uint32_t(sms * patch_ctas<FORM>());
     kern<<<unsigned(B.npatches), kPatchThreads, smem, s>>>(q);
     count_launch();
     check_cuda("patch apply launch");
@@ -451,14 +377,29 @@ void run_patch_apply(const PatchPlan& B, PatchArgs q, cudaStream_t s) {
 
 }  // namespace dev
 
-void launch_patch_apply(const Pattern& P, const dev::AsmParams& p, bool elas, bool kp1, bool fp32, const double* x,
-                        double* y, void* stream) {
-  const PatchPlan& B = patch_plan(P);
-  dev::PatchArgs q{};
+dev::PatchView patch_view(const PatchPlan& B, int ctas) {
+  dev::PatchView q{};
   q.hdr = B.d_hdr.as<PatchHdr>();
   q.conn = B.d_conn.as<uint16_t>();
   q.nodes = B.d_nodes.as<uint32_t>();
   q.chunks = B.d_chunks.as<uint4>();
+  q.partial = B.d_partial.as<double>();
+  q.npartial = B.npartial;
+  q.stride = B.stride;
+  q.nx = (B.max_nodes + 1) & ~1;  // (what lies behind starts on 16 bytes)
+  q.nv = B.max_verts;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  q.ahead = uint32_t(sms * ctas);
+  return q;
+}
+
+void launch_patch_apply(const Pattern& P, const dev::AsmParams& p, bool elas, bool kp1, bool fp32, const double* x,
+                        double* y, void* stream) {
+  const PatchPlan& B = patch_plan(P);
+  dev::PatchArgs q{};
+  static_cast<dev::PatchView&>(q) = patch_view(B, elas ? dev::patch_ctas<dev::FORM_ELAS>() : dev::patch_ctas<dev::FORM_DIFF>());
   q.xw = p.xw;
   q.kappa = kp1 ? p.kappa : nullptr;
   q.kscale = p.kscale;
@@ -480,12 +421,7 @@ void launch_patch_apply(const Pattern& P, const dev::AsmParams& p, bool elas, bo
   }
   q.x = x;
   q.y = y;
-  q.partial = B.d_partial.as<double>();
   q.nnodes = p.nnodes;
-  q.npartial = B.npartial;
-  q.stride = B.stride;
-  q.nx = (B.max_nodes + 1) & ~1;  // (the vertex records behind start on 16 bytes)
-  q.nv = B.max_verts;
   const int D = P.V->mesh->tdim, deg = P.V->degree;
   if (elas) {
     if (deg == 1) {
