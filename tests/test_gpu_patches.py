@@ -1,4 +1,5 @@
-"""Matrix-free action over cell patches against the oracle's CSR times x:
+"""Matrix-free action and load vector over cell patches.  The action against the
+oracle's CSR times x:
 one patch and many, patches that share nodes, ragged boxes, permuted vertex
 numbering, a vertex of no cell, and an x that is also y.  Row-wise bound:
 |y - R x| <= tol sum_j |R_ij x_j| with tol = 1e-12 (FP64: a row takes at most
@@ -110,3 +111,49 @@ def test_first_action_inside_a_graph_capture():
     torch.cuda.synchronize()
     ref = d2.assemble_action(a, d2.Vector(xv)).tensor()
     assert torch.equal(y.tensor(), ref)
+
+
+@pytest.mark.parametrize("dims,deg", [((14, 14, 14), 2), ((15, 15, 15), 2), ((20, 20, 20), 1), ((21, 21, 21), 1),
+                                      ((353, 353), 2), ((354, 354), 2)])
+@pytest.mark.parametrize("kind", ["p1", "const"])
+def test_load_vector_on_both_sides_of_the_patch_line(orc, dims, deg, kind):
+    """Tetrahedra change at 200,000 incidences (P2 n = 14 / 15, P1 n = 20 / 21),
+    triangles at 1.5 million (P2 n = 353 / 354); each entry against the oracle
+    (1e-12 of the largest), accumulation, and row ranges bit for bit."""
+    om = _mesh(orc, dims, False)
+    mesh = d2.Mesh(om.coords, om.cells)
+    V = d2.FunctionSpace(mesh, "Lagrange", deg)
+    v = d2.TestFunction(V)
+    od, N = orc.dofmap(om, deg, 1)
+    if kind == "p1":
+        fv = synthetic.uniform_field(om.nv, -1.0, 1.0, 11)
+        L = d2.Function(d2.FunctionSpace(mesh, "Lagrange", 1), fv) * v * d2.dx
+        ref = orc.assemble_vector(orc.form(orc.LOAD, len(dims), deg, 1, coeff=orc.COEFF_P1), om, od, N, w=fv)
+    else:
+        L = d2.Constant(-2.5) * v * d2.dx
+        ref = orc.assemble_vector(orc.form(orc.LOAD, len(dims), deg, 1, coeff=orc.COEFF_CONST, c=(-2.5,)), om, od, N)
+    b = d2.assemble(L)
+    got = b.get_local()
+    assert np.max(np.abs(got - ref)) <= 1e-12 * np.max(np.abs(ref))
+    d2.assemble(L, tensor=b, add_values=True)
+    assert np.allclose(b.get_local(), 2 * got, rtol=1e-15, atol=0)
+    P = V.pattern()
+    part = d2.Vector(torch.full((N,), float("nan"), dtype=torch.float64, device="cuda"))
+    try:
+        for a, e in ((0, om.nv // 3), (om.nv // 3, N - 5), (N - 5, N)):
+            P.set_row_range(a, e)
+            d2.assemble(L, tensor=part)
+    finally:
+        P.set_row_range(0, N)
+    assert np.array_equal(part.get_local(), got)
+
+
+def test_vector_load_over_patches(orc):
+    om = _mesh(orc, (15, 15, 15), False)
+    mesh = d2.Mesh(om.coords, om.cells)
+    V = d2.VectorFunctionSpace(mesh, "Lagrange", 2)
+    c = (0.5, 0.0, -1.5)
+    b = d2.assemble(d2.inner(d2.Constant(c), d2.TestFunction(V)) * d2.dx)
+    od, N = orc.dofmap(om, 2, 3)
+    ref = orc.assemble_vector(orc.form(orc.LOAD, 3, 2, 3, coeff=orc.COEFF_CONST, c=c), om, od, N)
+    assert np.max(np.abs(b.get_local() - ref)) <= 1e-12 * np.max(np.abs(ref))
