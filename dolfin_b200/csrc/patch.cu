@@ -109,7 +109,7 @@ __device__ __forceinline__ void p2_test_linear(const double (&F)[D + 1][D], cons
 template <int D, int P, int FORM, bool KP1, typename CT>
 __device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&xv)[D + 1][D],
                                             const double (&kap)[D + 1],
-                                            const double (&xc)[FORM == FORM_ELAS ? D : 1][El<D, P>::K],
+                                            const CT (&xc)[FORM == FORM_ELAS ? D : 1][El<D, P>::K],
                                             double (&y)[FORM == FORM_ELAS ? D : 1][El<D, P>::K]) {
   constexpr int NB = D + 1, K = El<D, P>::K, BS = FORM == FORM_ELAS ? D : 1;
   double g[NB][D];
@@ -189,7 +189,7 @@ __device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&x
   } else {
     // quadrature (P1: the centroid), in the contraction type
     using Q = Quad<D, P == 1 ? 1 : (FORM == FORM_ELAS ? 2 : 3)>;
-    CT gc[NB][D], xq[BS][K];
+    CT gc[NB][D];
 #pragma unroll
     for (int a = 0; a < NB; ++a)
 #pragma unroll
@@ -197,10 +197,7 @@ __device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&x
 #pragma unroll
     for (int e = 0; e < BS; ++e)
 #pragma unroll
-      for (int j = 0; j < K; ++j) {
-        xq[e][j] = CT(xc[e][j]);
-        y[e][j] = 0.0;
-      }
+      for (int j = 0; j < K; ++j) y[e][j] = 0.0;
 #pragma unroll
     for (int n = 0; n < Q::NQ; ++n) {
       double l[NB];
@@ -214,7 +211,7 @@ __device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&x
         for (int d = 0; d < D; ++d) gu[e][d] = CT(0);
 #pragma unroll
         for (int a = 0; a < NB; ++a) {
-          const CT u = node_derivative<D, P, CT>(xq[e], l, a);
+          const CT u = node_derivative<D, P, CT>(xc[e], l, a);
 #pragma unroll
           for (int d = 0; d < D; ++d) gu[e][d] = fma(u, gc[a][d], gu[e][d]);
         }
@@ -271,13 +268,14 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
   constexpr int NB = D + 1, K = El<D, P>::K, BS = FORM == FORM_ELAS ? D : 1;
   constexpr int T = kPatchThreads;
   extern __shared__ __align__(16) unsigned char smem[];
-  // the nodes' x by component, vertex records (x, y, z, kappa), the staged
-  // actions by component and local node (and a zero slot each), the jobs
-  double* xs = reinterpret_cast<double*>(smem);
-  double* vs = xs + BS * q.nx;
-  CT* ys = reinterpret_cast<CT*>(vs + 4 * q.nv);
+  // vertex records (x, y, z, kappa), the nodes' x by component (in the
+  // contraction type: one conversion a node, not one a cell and node), the
+  // staged actions by component and local node (and a zero slot each), the jobs
+  double* vs = reinterpret_cast<double*>(smem);
+  CT* xs = reinterpret_cast<CT*>(vs + 4 * q.nv);
+  CT* ys = xs + BS * q.nx;
   const int plane = K * q.stride + 1;
-  unsigned char* jobs = smem + PatchPlan::pad16(uint32_t((4 * q.nv + BS * q.nx) * 8 + BS * plane * int(sizeof(CT))));
+  unsigned char* jobs = smem + PatchPlan::pad16(uint32_t(32 * q.nv + BS * (q.nx + plane) * int(sizeof(CT))));
   const PatchHdr h = patch_header(q.hdr, blockIdx.x);
   // the plan data of a patch that starts later goes to L2 meanwhile (P2 tets
   // n=96 0.246 -> 0.230 ms)
@@ -291,7 +289,7 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
   for (int i = threadIdx.x; i < h.nnodes; i += T) {
     const uint32_t node = __ldg(q.nodes + h.node0 + i);
 #pragma unroll
-    for (int e = 0; e < BS; ++e) xs[e * q.nx + i] = __ldg(q.x + int64_t(e) * q.nnodes + node);
+    for (int e = 0; e < BS; ++e) xs[e * q.nx + i] = CT(__ldg(q.x + int64_t(e) * q.nnodes + node));
     if (i < h.nverts) {
       double a, b, c, d;
       ld_rec4(q.xw + 4 * size_t(node), a, b, c, d);
@@ -305,7 +303,8 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
   __syncthreads();
   if (later < gridDim.x) patch_prefetch<K>(q, hn);
   for (int c = threadIdx.x; c < h.ncells; c += T) {
-    double xv[NB][D], kap[NB], xc[BS][K], y[BS][K];
+    double xv[NB][D], kap[NB], y[BS][K];
+    CT xc[BS][K];
 #pragma unroll
     for (int a = 0; a < NB; ++a) {
       const double2* v = reinterpret_cast<const double2*>(reinterpret_cast<const char*>(vs) + 4 * cn.off(a));
@@ -317,9 +316,9 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
     }
 #pragma unroll
     for (int j = 0; j < K; ++j) {
-      const char* xj = reinterpret_cast<const char*>(xs) + cn.off(j);
+      const char* xj = reinterpret_cast<const char*>(xs) + (sizeof(CT) == 8 ? cn.off(j) : cn.off(j) / 2u);
 #pragma unroll
-      for (int e = 0; e < BS; ++e) xc[e][j] = reinterpret_cast<const double*>(xj)[e * q.nx];
+      for (int e = 0; e < BS; ++e) xc[e][j] = reinterpret_cast<const CT*>(xj)[e * q.nx];
     }
     if (c + T < h.ncells) cn.load(q, h, c + T);
     cell_action<D, P, FORM, KP1, CT>(q, xv, kap, xc, y);
@@ -361,7 +360,7 @@ void run_patch_apply(const PatchPlan& B, const PatchArgs& q, cudaStream_t s) {
     auto kern = k_patch_apply<D, P, FORM, KP1, CT>;
     static unsigned long long configured = 0;
     allow_dynamic_smem(kern, configured);
-    const size_t smem = PatchPlan::pad16(uint32_t((4 * q.nv + BS * q.nx) * 8 + BS * (K * q.stride + 1) * int(sizeof(CT)))) +
+    const size_t smem = PatchPlan::pad16(uint32_t(32 * q.nv + BS * (q.nx + K * q.stride + 1) * int(sizeof(CT)))) +
                         size_t(B.max_chunks) * 16;
     kern<<<unsigned(B.npatches), kPatchThreads, smem, s>>>(q);
     count_launch();
