@@ -271,7 +271,7 @@ int db2_batch_info(db2_batch B, int64_t* tiles, int64_t* cells, int* ctas) {
   });
 }
 
-// The persistent launch (counter reset, kappa packing, assembly) is captured
+// The persistent launch (kappa packing with the counter reset, assembly) is captured
 // into a CUDA graph on first use per precision and replayed on `stream`.
 int db2_batch_assemble(db2_batch Bh, int precision, void* stream) {
   return db2::guard_call([&] {

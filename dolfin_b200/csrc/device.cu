@@ -75,6 +75,50 @@ void PlanUpload::put(DeviceBuffer& d, const void* host, size_t nbytes) {
   if (e != cudaSuccess) fail(DB2_ERR_CUDA, "plan upload: %s", cudaGetErrorString(e));
 }
 
+// (pool calls stay out of a capture that another stream of the thread is in)
+StreamScratch::~StreamScratch() {
+  if (!pool_) return;
+  cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&m);
+  cudaMemPoolDestroy(static_cast<cudaMemPool_t>(pool_));
+  cudaThreadExchangeStreamCaptureMode(&m);
+}
+
+void* StreamScratch::take(size_t nbytes, void* stream) const {
+  if (nbytes == 0) return nullptr;
+  cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&m);
+  cudaError_t e = cudaSuccess;
+  void* ptr = nullptr;
+  {
+    std::lock_guard<std::mutex> guard(lock_);
+    if (!pool_) {
+      cudaMemPoolProps props{};
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      e = cudaGetDevice(&props.location.id);
+      cudaMemPool_t pool = nullptr;
+      if (e == cudaSuccess) e = cudaMemPoolCreate(&pool, &props);
+      uint64_t keep = UINT64_MAX;  // no return to the driver at each synchronisation
+      if (e == cudaSuccess) e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+      pool_ = pool;
+    }
+    if (e == cudaSuccess)
+      e = cudaMallocFromPoolAsync(&ptr, nbytes, static_cast<cudaMemPool_t>(pool_), static_cast<cudaStream_t>(stream));
+  }
+  cudaThreadExchangeStreamCaptureMode(&m);
+  if (e != cudaSuccess) fail(DB2_ERR_CUDA, "call scratch of %zu bytes: %s", nbytes, cudaGetErrorString(e));
+  return ptr;
+}
+
+void StreamScratch::give(void* ptr, void* stream) const {
+  if (!ptr) return;
+  cudaStreamCaptureMode m = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&m);
+  cudaFreeAsync(ptr, static_cast<cudaStream_t>(stream));
+  cudaThreadExchangeStreamCaptureMode(&m);
+}
+
 // Vertex records of 4 doubles -- (x, y, z, kappa) in 3D, (x, y, kappa, f) in
 // 2D -- so that a vertex is one aligned 256-bit load; the coefficient slots
 // are written per assembly call (pack_vertex_records).

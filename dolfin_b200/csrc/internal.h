@@ -2,8 +2,10 @@
 #pragma once
 
 #include <algorithm>
+#include <array>
 #include <cstdint>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -63,6 +65,21 @@ struct PlanUpload {
  private:
   void* stream_ = nullptr;
   int mode_;
+};
+
+// Scratch of one call, ordered by its stream: calls of several streams and
+// threads each have their own.  The driver's stream-ordered pool keeps what was
+// given back (a call's worth for each stream in use at once) until the owner goes.
+struct StreamScratch {
+  StreamScratch() = default;
+  StreamScratch(const StreamScratch&) = delete;
+  StreamScratch& operator=(const StreamScratch&) = delete;
+  ~StreamScratch();
+  void* take(size_t nbytes, void* stream) const;  // null for 0 bytes
+  void give(void* ptr, void* stream) const;       // after the last launch using it
+ private:
+  mutable std::mutex lock_;
+  mutable void* pool_ = nullptr;
 };
 
 // ---- mesh ----------------------------------------------------------------
@@ -185,6 +202,12 @@ struct PatchPlan {
   std::vector<uint32_t> shared_ptr;  // their partial slots, in patch order
   DeviceBuffer d_hdr, d_conn, d_nodes, d_chunks, d_shared, d_shared_ptr, d_partial;
   DeviceBuffer d_x;              // copy of an x that shares memory with y
+  StreamScratch scratch;         // a load vector's partial sums
+  // per patch: its vertex nodes lie in [b[0], b[1]], its edge nodes in [b[2], b[3]]
+  std::vector<std::array<uint32_t, 4>> bounds;
+  // patches meeting the row range they were listed for
+  mutable int64_t list_begin = -1, list_end = -1, list_size = 0;
+  mutable DeviceBuffer d_list;
   static constexpr uint32_t pad16(uint32_t n) { return (n + 15u) & ~15u; }
 };
 
@@ -241,7 +264,8 @@ struct Pattern {
   ReorderedCSR reordered;
   std::unique_ptr<FacetPlan> facets;
   const FacetPlan& facet_plan();     // built and uploaded on first use
-  mutable std::unique_ptr<PatchPlan> patches;
+  mutable std::mutex patches_lock;
+  mutable std::unique_ptr<PatchPlan> patches;  // built on first use (patch_plan)
 };
 
 // Relabelling of a cell so that local node `li` becomes canonical: for a
@@ -277,6 +301,9 @@ void build_facet_plan(Pattern& P);
 std::unique_ptr<PatchPlan> make_patches(const Pattern& P, int max_cells);
 // The pattern's patches, built and uploaded on first use.
 const PatchPlan& patch_plan(const Pattern& P);
+// How many patches the pattern's row range needs, and their numbers on the
+// device (null: all of them).  After patch_plan(P).
+int64_t patches_of_rows(const Pattern& P, const uint32_t** list);
 // Re-cut the tiles of an existing plan (autotuning), re-uploading d_tiles.
 void retile(Pattern& P, int tile_threads, int seg_cap_bytes);
 // Tiles of a pattern for a launch shape (pure; does not modify P).

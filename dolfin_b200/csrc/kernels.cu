@@ -4,7 +4,7 @@
 #include "launch.cuh"
 
 namespace db2 {
-void launch_patch_load(const Pattern& P, const dev::AsmParams& p, int loadm, void* stream);
+bool launch_patch_load(const Pattern& P, const dev::AsmParams& p, int loadm, void* stream);  // false: not taken
 
 namespace dev {
 
@@ -158,9 +158,12 @@ static bool latency_bound(const Pattern& P, bool fp32) {
 // or by the thread-per-row kernel (one launch, in 2D after a packing one).
 // Measured on B200 (us a call, by rows -> over patches): P2 tets n=10 (60,000
 // incidences) 17 -> 18, n=16 (245,760) 18 -> 15, n=34 33 -> 18, n=50 80 -> 38,
-// n=72 227 -> 93, n=96 533 -> 210; P1 tets n=20 (192,000) 15 -> 20, n=40 17 ->
+// n=72 227 -> 93, n=96 430 -> 193; P1 tets n=20 (192,000) 15 -> 20, n=40 17 ->
 // 15, n=60 55 -> 31; P2 triangles n=200 (480,000) 14 -> 15, 500x300 (1.8 M) 22.4
 // -> 21.8.
+// One eighth of P2 n=96's rows (set_row_range): 49 -> 43-56; the eighth
+// that holds the vertices, which meet every patch, 149 -> 187, kept so that a share
+// of the rows equals the whole vector's bit for bit.
 static bool load_over_patches(const Pattern& P) {
   return int64_t(P.inc.size()) >= (P.V->mesh->tdim == 3 ? 200000 : 1500000);
 }
@@ -189,10 +192,7 @@ void launch_assemble(const Pattern& P, const FormArgs* a, const FormArgs* L, int
   if (!a) {
     // rank-1 form only
     if (loadm == dev::LOAD_NONE) fail(DB2_ERR_ARGUMENT, "nothing to assemble");
-    if (load_over_patches(P)) {
-      launch_patch_load(P, p, loadm, stream);
-      return;
-    }
+    if (load_over_patches(P) && launch_patch_load(P, p, loadm, stream)) return;
     pack_vertex_records(P, nullptr, loadm == dev::LOAD_P1 ? p.f : nullptr, stream);
     // the node rows of the pattern's row range (all of them by default)
     const int64_t n0 = P.row_begin, nr = (P.row_end < 0 ? V.nnodes : P.row_end) - n0;

@@ -11,7 +11,7 @@
 // (60 B a cell), x, y and about one partial sum a cell.  Measured on B200, ms
 // per action: vector P2 elasticity n=48 0.245 -> 0.087, P2 tets n=96 0.342 ->
 // 0.230, P1 tets n=80 0.102 -> 0.060; with FP32 actions 63x70x57 0.084 ->
-// 0.081 (its quadrature is unchanged, and issue-bound).
+// 0.079 (its quadrature is unchanged, and issue-bound).
 #include <cuda_runtime.h>
 
 #include "patch.cuh"

@@ -16,6 +16,7 @@ namespace dev {
 struct PatchLoadArgs : PatchView {
   int bs;
   uint32_t row_begin, row_end;  // node rows to assemble
+  const uint32_t* list;         // the patches that may hold some of them; null: all
 };
 
 template <int D, int P, int LOADM, int LI>
@@ -57,10 +58,11 @@ __global__ void __launch_bounds__(kLoadThreads, 5) k_patch_load(const AsmParams 
   double* vs = reinterpret_cast<double*>(smem);
   double* ys = vs + 4 * q.nv;
   unsigned char* jobs = smem + PatchPlan::pad16(uint32_t((4 * q.nv + K * q.stride + 1) * 8));
-  const PatchHdr h = patch_header(q.hdr, blockIdx.x);
+  auto patch = [&](uint32_t i) { return q.list ? __ldg(q.list + i) : i; };
+  const PatchHdr h = patch_header(q.hdr, patch(blockIdx.x));
   const uint32_t later = blockIdx.x + q.ahead;
   PatchHdr hn{};
-  if (later < gridDim.x) hn = patch_header(q.hdr, later);
+  if (later < gridDim.x) hn = patch_header(q.hdr, patch(later));
   patch_jobs_copy(q, h, jobs);
   PatchCell<K> cn{};
   if (int(threadIdx.x) < h.ncells) cn.load(q, h, threadIdx.x);
@@ -128,16 +130,18 @@ __global__ void __launch_bounds__(256) k_patch_load_sum(const AsmParams p, const
 }
 
 template <int D, int P, int LOADM>
-void run_patch_load(const PatchPlan& B, const AsmParams& p, const PatchLoadArgs& q, cudaStream_t s) {
+void run_patch_load(const PatchPlan& B, int64_t npatches, const AsmParams& p, const PatchLoadArgs& q, cudaStream_t s) {
   constexpr int K = El<D, P>::K;
   auto kern = k_patch_load<D, P, LOADM>;
   static unsigned long long configured = 0;
   allow_dynamic_smem(kern, configured);
   const size_t smem =
       PatchPlan::pad16(uint32_t((4 * q.nv + K * q.stride + 1) * 8)) + size_t(B.max_chunks) * 16;
-  kern<<<unsigned(B.npatches), kLoadThreads, smem, s>>>(p, q);
-  count_launch();
-  check_cuda("patch load launch");
+  if (npatches > 0) {
+    kern<<<unsigned(npatches), kLoadThreads, smem, s>>>(p, q);
+    count_launch();
+    check_cuda("patch load launch");
+  }
   if (B.nshared > 0) {
     k_patch_load_sum<LOADM><<<unsigned((B.nshared + 255) / 256), 256, 0, s>>>(
         p, q, B.d_shared.as<uint32_t>(), B.d_shared_ptr.as<uint32_t>(), B.nshared);
@@ -148,23 +152,50 @@ void run_patch_load(const PatchPlan& B, const AsmParams& p, const PatchLoadArgs&
 
 }  // namespace dev
 
-void launch_patch_load(const Pattern& P, const dev::AsmParams& p, int loadm, void* stream) {
-  const PatchPlan& B = patch_plan(P);
+bool launch_patch_load(const Pattern& P, const dev::AsmParams& p, int loadm, void* stream) {
   cudaStream_t s = static_cast<cudaStream_t>(stream);
+  // A graph's replays may overlap one another and later calls, so a captured
+  // call would need partial sums of its own for the graph's life.
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return false;
+  }
+  const PatchPlan* plan = nullptr;
+  void* partial = nullptr;
+  int64_t npatches = 0;
+  const uint32_t* list = nullptr;
+  try {
+    plan = &patch_plan(P);
+    npatches = patches_of_rows(P, &list);
+    partial = plan->scratch.take(size_t(plan->npartial) * sizeof(double), stream);
+  } catch (const Error&) {  // no room for the plan or the partial sums
+    cudaGetLastError();
+    return false;
+  }
+  struct Give {
+    const StreamScratch& pool;
+    void *ptr, *stream;
+    ~Give() { pool.give(ptr, stream); }
+  } give{plan->scratch, partial, stream};
+  const PatchPlan& B = *plan;
   const int D = P.V->mesh->tdim, deg = P.V->degree;
   dev::PatchLoadArgs q{};
   static_cast<dev::PatchView&>(q) = patch_view(B, 5);
+  q.partial = static_cast<double*>(partial);
   q.bs = P.bs;
   q.row_begin = uint32_t(P.row_begin);
   q.row_end = uint32_t(P.row_end < 0 ? P.V->nnodes : P.row_end);
+  q.list = list;
 #define DB2_PL(D_, P_)                                                                           \
   if (D == D_ && deg == P_) {                                                                    \
-    if (loadm == dev::LOAD_CONST) dev::run_patch_load<D_, P_, dev::LOAD_CONST>(B, p, q, s);      \
-    else dev::run_patch_load<D_, P_, dev::LOAD_P1>(B, p, q, s);                                  \
-    return;                                                                                      \
+    if (loadm == dev::LOAD_CONST) dev::run_patch_load<D_, P_, dev::LOAD_CONST>(B, npatches, p, q, s);      \
+    else dev::run_patch_load<D_, P_, dev::LOAD_P1>(B, npatches, p, q, s);                                  \
+    return true;                                                                                 \
   }
   DB2_PL(3, 1) DB2_PL(3, 2) DB2_PL(2, 1) DB2_PL(2, 2)
 #undef DB2_PL
+  return false;
 }
 
 }  // namespace db2

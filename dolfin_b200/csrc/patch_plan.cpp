@@ -339,9 +339,18 @@ std::unique_ptr<PatchPlan> make_patches(const Pattern& P, int max_cells) {
 // Small meshes are cut into about 600 patches (four for each of 148 SMs), down
 // to 64 cells: one patch's latency is the action's.
 const PatchPlan& patch_plan(const Pattern& P) {
+  std::lock_guard<std::mutex> guard(P.patches_lock);
   if (!P.patches) {
     const int full = P.V->degree == 1 ? 512 : P.bs > 1 ? 200 : 330;
     auto B = make_patches(P, int(std::min<int64_t>(full, std::max<int64_t>(64, P.V->mesh->nc / 592))));
+    for (const PatchHdr& h : B->hdr) {  // (a patch's nodes ascend, vertices first)
+      std::array<uint32_t, 4> b{1, 0, 1, 0};  // empty
+      const uint32_t* n = B->nodes.data() + h.node0;
+      const int k = h.nverts;
+      if (k > 0) b[0] = n[0], b[1] = n[k - 1];
+      if (k < h.nnodes) b[2] = n[k], b[3] = n[h.nnodes - 1];
+      B->bounds.push_back(b);
+    }
     PlanUpload U;
     auto up = [&](DeviceBuffer& d, auto& v) {
       if (!v.empty()) U.put(d, v.data(), v.size() * sizeof(v[0]));
@@ -357,6 +366,29 @@ const PatchPlan& patch_plan(const Pattern& P) {
     P.patches = std::move(B);
   }
   return *P.patches;
+}
+
+int64_t patches_of_rows(const Pattern& P, const uint32_t** list) {
+  const PatchPlan& B = *P.patches;
+  const int64_t r0 = P.row_begin, r1 = P.row_end < 0 ? P.V->nnodes : P.row_end;
+  *list = nullptr;
+  if (r0 == 0 && r1 == P.V->nnodes) return B.npatches;
+  if (r0 >= r1) return 0;
+  std::lock_guard<std::mutex> guard(P.patches_lock);
+  if (B.list_begin != r0 || B.list_end != r1) {
+    std::vector<uint32_t> ids;
+    auto meets = [&](uint32_t a, uint32_t b) { return a <= b && a < r1 && b >= r0; };
+    for (size_t i = 0; i < B.bounds.size(); ++i)
+      if (meets(B.bounds[i][0], B.bounds[i][1]) || meets(B.bounds[i][2], B.bounds[i][3])) ids.push_back(uint32_t(i));
+    B.list_begin = -1;
+    PlanUpload U;
+    U.put(B.d_list, ids.data(), ids.size() * sizeof(uint32_t));
+    B.list_size = int64_t(ids.size());
+    B.list_begin = r0;
+    B.list_end = r1;
+  }
+  *list = B.d_list.as<uint32_t>();
+  return B.list_size;
 }
 
 }  // namespace db2

@@ -157,3 +157,32 @@ def test_vector_load_over_patches(orc):
     od, N = orc.dofmap(om, 2, 3)
     ref = orc.assemble_vector(orc.form(orc.LOAD, 3, 2, 3, coeff=orc.COEFF_CONST, c=c), om, od, N)
     assert np.max(np.abs(b.get_local() - ref)) <= 1e-12 * np.max(np.abs(ref))
+
+
+def test_load_vectors_on_several_streams_and_under_capture():
+    """Calls on one pattern that overlap (four streams) have partial sums of
+    their own: each equals the lone call bit for bit.  A captured call sums by
+    rows (1e-13 of the largest: ~120 terms a row)."""
+    V = d2.FunctionSpace(d2.UnitCubeMesh(24, 24, 24), "Lagrange", 2)
+    v = d2.TestFunction(V)
+    Ls = [d2.Constant(c) * v * d2.dx for c in (1.0, -3.0, 0.5, 7.0)]
+    alone = [d2.assemble(L).get_local() for L in Ls]
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in Ls]
+    outs = [[d2.Vector(n=V.dim()) for _ in range(8)] for _ in Ls]
+    torch.cuda.synchronize()
+    for r in range(8):
+        for s, L, out in zip(streams, Ls, outs):
+            with torch.cuda.stream(s):
+                d2.assemble(L, tensor=out[r])
+    torch.cuda.synchronize()
+    for ref, out in zip(alone, outs):
+        for b in out:
+            assert np.array_equal(b.get_local(), ref)
+    b = d2.Vector(n=V.dim())
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        d2.assemble(Ls[1], tensor=b)
+    g.replay()
+    torch.cuda.synchronize()
+    assert np.max(np.abs(b.get_local() - alone[1])) <= 1e-13 * np.max(np.abs(alone[1]))
