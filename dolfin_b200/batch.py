@@ -3,7 +3,7 @@ captured launch (db2_batch_* in the C ABI), and its autotuner.
 
 Every member assembles kappa*inner(grad(u), grad(v))*dx on its own space
 (P1 or P2, triangles or tetrahedra) with its own P1 kappa.  ``assemble()``
-replays one captured graph (counter reset, kappa packing, one persistent
+replays one captured graph (kappa packing and counter reset, one persistent
 kernel over all tiles); ``assemble_loop()`` is the reference: one launch per
 member.
 """

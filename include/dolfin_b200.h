@@ -291,10 +291,11 @@ int db2_assemble_facets_bc(db2_pattern P, const db2_form* a_ds, const double* wa
                            const double* bc_vals, double* vals, double* b, void* stream);
 /* Matrix-free action y = A(a) x (device x[N], y[N]); replaces assembling A
    and calling GenericMatrix::mult (dolfin/la/GenericMatrix.h).  Computed
-   per cell (element actions, exact quadrature) and summed per row in cell
-   order, so repeated calls agree bitwise.  The first call on a pattern
-   allocates cells * bs * k doubles of device work space, kept by the
-   pattern; calls on one pattern that overlap on the GPU race on it. */
+   per cell (element actions, exact integration) and summed per row in a
+   fixed order, so repeated calls agree bitwise; x and y may be one array.
+   The first call on a pattern builds its cell patches (plan arrays of about
+   60 bytes a cell and one partial sum a cell on the device, kept by the
+   pattern); calls on one pattern that overlap on the GPU race on them. */
 int db2_apply(db2_pattern P, const db2_form* a, const double* w, int precision, const double* x,
               double* y, void* stream);
 /* db2_apply with DB2_FP32_CONTRACT computes the element actions in FP32
