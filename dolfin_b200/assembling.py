@@ -273,15 +273,24 @@ def assemble_action(a, x, y=None, precision="fp64"):
 
 def _bc_arrays(V, bcs):
     """Dirichlet flags and values over the dofs, from the conditions' dofs and
-    values kept on the device (copying them from the host at every call cost
-    about 100 us and a synchronisation)."""
+    values on the device.  A condition is anything with dofs_and_values()."""
     import torch
     flags = torch.zeros(V.dim(), dtype=torch.uint8, device="cuda")
     vals = torch.zeros(V.dim(), dtype=torch.float64, device="cuda")
     for bc in bcs:
-        dofs, values = bc.device_dofs_and_values()
-        for t in (dofs, values):  # they may have been made on another stream
-            t.record_stream(torch.cuda.current_stream())
-        flags.index_fill_(0, dofs, 1)
-        vals.index_copy_(0, dofs, values)
+        if hasattr(bc, "device_dofs_and_values"):
+            dofs, values, plain = bc.device_dofs_and_values()
+            for t in (dofs, values):  # they may have been made on another stream
+                t.record_stream(torch.cuda.current_stream())
+        else:
+            dofs, values = bc.dofs_and_values()
+            dofs = torch.as_tensor(dofs, dtype=torch.int64, device="cuda")
+            values = torch.as_tensor(values, dtype=torch.float64, device="cuda")
+            plain = False
+        if plain:
+            flags.index_fill_(0, dofs, 1)
+            vals.index_copy_(0, dofs, values)
+        else:
+            flags[dofs] = 1
+            vals[dofs] = values
     return flags, vals
