@@ -325,11 +325,11 @@ class SparsityPattern(_Handle):
         share of a row-partitioned assembly; see db2_pattern_set_row_range)."""
         call("db2_pattern_set_row_range", self._h, int(node_begin), int(node_end))
         self._block = False
-        self._range = (int(node_begin), int(node_end)) != (0, self.V.dim() // self.V.value_size())
 
     def has_row_range(self):
-        """Whether assemblies write only a part of the rows."""
-        return getattr(self, "_range", False) or self.holds_row_block()
+        """Whether assemblies write only a part of the rows (as the engine has
+        it: a range may also be set through the C entry points)."""
+        return self.row_block_info()[0] != self.nrows
 
     def set_row_block(self, node_begin, node_end):
         """As set_row_range, with the tensors holding the row block alone
