@@ -75,6 +75,22 @@ void PlanUpload::put(DeviceBuffer& d, const void* host, size_t nbytes) {
   if (e != cudaSuccess) fail(DB2_ERR_CUDA, "plan upload: %s", cudaGetErrorString(e));
 }
 
+bool stream_is_capturing(void* stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(static_cast<cudaStream_t>(stream), &status) != cudaSuccess) {
+    cudaGetLastError();
+    return true;
+  }
+  return status != cudaStreamCaptureStatusNone;
+}
+
+unsigned long long stream_id(void* stream) {
+  unsigned long long id = 0;
+  if (cudaStreamGetId(static_cast<cudaStream_t>(stream), &id) == cudaSuccess) return id;
+  cudaGetLastError();
+  return 0;
+}
+
 // (pool calls stay out of a capture that another stream of the thread is in)
 StreamScratch::~StreamScratch() {
   if (!pool_) return;
@@ -107,7 +123,11 @@ void* StreamScratch::take(size_t nbytes, void* stream) const {
       e = cudaMallocFromPoolAsync(&ptr, nbytes, static_cast<cudaMemPool_t>(pool_), static_cast<cudaStream_t>(stream));
   }
   cudaThreadExchangeStreamCaptureMode(&m);
-  if (e != cudaSuccess) fail(DB2_ERR_CUDA, "call scratch of %zu bytes: %s", nbytes, cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    fail(e == cudaErrorMemoryAllocation ? DB2_ERR_NOMEM : DB2_ERR_CUDA, "call scratch of %zu bytes: %s", nbytes,
+         cudaGetErrorString(e));
+  }
   return ptr;
 }
 

@@ -82,6 +82,12 @@ struct StreamScratch {
   mutable void* pool_ = nullptr;
 };
 
+// Whether the stream is being captured into a graph (or may not be used while
+// another one is).
+bool stream_is_capturing(void* stream);
+// An id that no other stream of the process has had or will have; 0 if there is none.
+unsigned long long stream_id(void* stream);
+
 // ---- mesh ----------------------------------------------------------------
 struct Mesh {
   int tdim = 0;
@@ -200,9 +206,21 @@ struct PatchPlan {
   std::vector<uint8_t> chunks;   // per patch: destinations (32 a group), groups, codes
   std::vector<uint32_t> shared;  // nodes with partial sums
   std::vector<uint32_t> shared_ptr;  // their partial slots, in patch order
-  DeviceBuffer d_hdr, d_conn, d_nodes, d_chunks, d_shared, d_shared_ptr, d_partial;
-  DeviceBuffer d_x;              // copy of an x that shares memory with y
-  StreamScratch scratch;         // a load vector's partial sums
+  DeviceBuffer d_hdr, d_conn, d_nodes, d_chunks, d_shared, d_shared_ptr;
+  // Work space of calls (CallScratch): partial sums, and copies of inputs that
+  // share memory with the output.  Kept for the first kStreams streams that
+  // calls come on, by the stream's id, which no later stream gets again; in a
+  // stream-ordered pool for calls on others.  `captured` is that of captured
+  // actions, whose graphs may be replayed at any time; it never moves.
+  struct Work {
+    unsigned long long stream_id = 0;
+    std::mutex busy;  // held from a call's first launch to its last
+    DeviceBuffer partial, x;
+  };
+  static constexpr size_t kStreams = 8;
+  mutable std::vector<std::unique_ptr<Work>> works;
+  mutable Work captured;
+  StreamScratch scratch;
   // per patch: its vertex nodes lie in [b[0], b[1]], its edge nodes in [b[2], b[3]]
   std::vector<std::array<uint32_t, 4>> bounds;
   // patches meeting the row range they were listed for
@@ -301,6 +319,22 @@ void build_facet_plan(Pattern& P);
 std::unique_ptr<PatchPlan> make_patches(const Pattern& P, int max_cells);
 // The pattern's patches, built and uploaded on first use.
 const PatchPlan& patch_plan(const Pattern& P);
+// Work space of one call over the pattern's patches, from before its first
+// launch until behind its last.  Calls on one stream and pattern take turns.
+class CallScratch {
+ public:
+  CallScratch(const Pattern& P, void* stream);
+  ~CallScratch();
+  CallScratch(const CallScratch&) = delete;
+  CallScratch& operator=(const CallScratch&) = delete;
+  double* take(DeviceBuffer PatchPlan::Work::*which, int64_t n);  // each at most once
+ private:
+  const Pattern& P_;
+  void* stream_;
+  PatchPlan::Work* work_ = nullptr;  // null: the pool
+  std::unique_lock<std::mutex> busy_;
+  std::vector<void*> taken_;
+};
 // How many patches the pattern's row range needs, and their numbers on the
 // device (null: all of them).  After patch_plan(P).
 int64_t patches_of_rows(const Pattern& P, const uint32_t** list);

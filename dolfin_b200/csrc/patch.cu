@@ -382,7 +382,6 @@ dev::PatchView patch_view(const PatchPlan& B, int ctas) {
   q.conn = B.d_conn.as<uint16_t>();
   q.nodes = B.d_nodes.as<uint32_t>();
   q.chunks = B.d_chunks.as<uint4>();
-  q.partial = B.d_partial.as<double>();
   q.npartial = B.npartial;
   q.stride = B.stride;
   q.nx = (B.max_nodes + 1) & ~1;  // (what lies behind starts on 16 bytes)
@@ -406,17 +405,15 @@ void launch_patch_apply(const Pattern& P, const dev::AsmParams& p, bool elas, bo
   q.lmbda = p.lmbda;
   const int64_t n = P.V->dim();
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // a patch writes its finished nodes while others still read x: an x that
-  // shares memory with y is copied first
+  CallScratch work(P, stream);
+  q.partial = work.take(&PatchPlan::Work::partial, B.npartial * P.bs);
+  // a patch writes its finished nodes while others still read x, and reads it
+  // through the read-only path: an x that shares memory with y is copied first
   if (x < y + n && y < x + n) {
-    DeviceBuffer& c = const_cast<PatchPlan&>(B).d_x;
-    if (c.bytes < size_t(n) * sizeof(double)) {
-      PlanUpload scope;
-      c.alloc(size_t(n) * sizeof(double));
-    }
-    cudaMemcpyAsync(c.ptr, x, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
+    double* c = work.take(&PatchPlan::Work::x, n);
+    cudaMemcpyAsync(c, x, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
     check_cuda("copy of x");
-    x = c.as<double>();
+    x = c;
   }
   q.x = x;
   q.y = y;

@@ -6,6 +6,7 @@
 // rebuilds every incident cell's geometry -- ten times a cell for P2 tetrahedra.
 #include <cuda_runtime.h>
 
+#include <optional>
 #include <utility>
 
 #include "patch.cuh"
@@ -156,33 +157,25 @@ bool launch_patch_load(const Pattern& P, const dev::AsmParams& p, int loadm, voi
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   // A graph's replays may overlap one another and later calls, so a captured
   // call would need partial sums of its own for the graph's life.
-  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(s, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone) {
-    cudaGetLastError();
-    return false;
-  }
-  const PatchPlan* plan = nullptr;
-  void* partial = nullptr;
+  if (stream_is_capturing(stream)) return false;
+  std::optional<CallScratch> work;
+  double* partial = nullptr;
   int64_t npatches = 0;
   const uint32_t* list = nullptr;
   try {
-    plan = &patch_plan(P);
+    const PatchPlan& B = patch_plan(P);
     npatches = patches_of_rows(P, &list);
-    partial = plan->scratch.take(size_t(plan->npartial) * sizeof(double), stream);
+    work.emplace(P, stream);
+    partial = work->take(&PatchPlan::Work::partial, B.npartial);
   } catch (const Error&) {  // no room for the plan or the partial sums
     cudaGetLastError();
     return false;
   }
-  struct Give {
-    const StreamScratch& pool;
-    void *ptr, *stream;
-    ~Give() { pool.give(ptr, stream); }
-  } give{plan->scratch, partial, stream};
-  const PatchPlan& B = *plan;
+  const PatchPlan& B = *P.patches;
   const int D = P.V->mesh->tdim, deg = P.V->degree;
   dev::PatchLoadArgs q{};
   static_cast<dev::PatchView&>(q) = patch_view(B, 5);
-  q.partial = static_cast<double*>(partial);
+  q.partial = partial;
   q.bs = P.bs;
   q.row_begin = uint32_t(P.row_begin);
   q.row_end = uint32_t(P.row_end < 0 ? P.V->nnodes : P.row_end);

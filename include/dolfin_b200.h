@@ -293,9 +293,12 @@ int db2_assemble_facets_bc(db2_pattern P, const db2_form* a_ds, const double* wa
    and calling GenericMatrix::mult (dolfin/la/GenericMatrix.h).  Computed
    per cell (element actions, exact integration) and summed per row in a
    fixed order, so repeated calls agree bitwise; x and y may be one array.
-   The first call on a pattern builds its cell patches (plan arrays of about
-   60 bytes a cell and one partial sum a cell on the device, kept by the
-   pattern); calls on one pattern that overlap on the GPU race on them. */
+   The first call on a pattern builds its cell patches (plan arrays of 50 to
+   100 bytes a cell on the device, kept by the pattern).  Partial sums,
+   about one a cell and component, are kept for each of the first eight
+   streams that calls come on and come from a stream-ordered pool on others, so
+   calls may overlap on several streams and threads; captured calls share one
+   set, so replays of their graphs must not overlap one another. */
 int db2_apply(db2_pattern P, const db2_form* a, const double* w, int precision, const double* x,
               double* y, void* stream);
 /* db2_apply with DB2_FP32_CONTRACT computes the element actions in FP32
