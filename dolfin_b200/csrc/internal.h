@@ -40,6 +40,11 @@ void parallel_for(int64_t n, F&& f, int64_t min_chunk = 4096) {
   for (auto& t : th) t.join();
 }
 
+// Whether n doubles at a and m doubles at b share memory (NULL: none).
+inline bool overlap(const double* a, int64_t n, const double* b, int64_t m) {
+  return a && b && a < b + m && b < a + n;
+}
+
 // Device buffer with RAII release (cudaFree); defined in device.cu.
 struct DeviceBuffer {
   void* ptr = nullptr;
@@ -215,7 +220,7 @@ struct PatchPlan {
   struct Work {
     unsigned long long stream_id = 0;
     std::mutex busy;  // held from a call's first launch to its last
-    DeviceBuffer partial, x;
+    DeviceBuffer partial, x, kappa;
   };
   static constexpr size_t kStreams = 8;
   mutable std::vector<std::unique_ptr<Work>> works;

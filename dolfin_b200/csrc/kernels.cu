@@ -168,6 +168,17 @@ static bool load_over_patches(const Pattern& P) {
   return int64_t(P.inc.size()) >= (P.V->mesh->tdim == 3 ? 200000 : 1500000);
 }
 
+// Whether the call writes over the memory of its kappa or f.  The tile classes
+// and the row kernel have copied them to the vertex records before they write
+// (f on triangles only); what reads the arrays beside its writes must not run.
+static bool writes_coefficients(const Pattern& P, const dev::AsmParams& p) {
+  int64_t nrows = P.nrows, nnz = P.nnz;
+  if (P.block_storage) row_block_size(P, &nrows, &nnz);
+  const int64_t nv = P.V->mesh->nv;
+  return overlap(p.b, nrows, p.kappa, nv) || overlap(p.b, nrows, p.f, nv) || overlap(p.vals, nnz, p.kappa, nv) ||
+         overlap(p.vals, nnz, p.f, nv);
+}
+
 void launch_assemble(const Pattern& P, const FormArgs* a, const FormArgs* L, int precision,
                      double* vals, double* b, bool add_values, const uint8_t* bc_flags,
                      const double* bc_vals, void* stream) {
@@ -192,7 +203,7 @@ void launch_assemble(const Pattern& P, const FormArgs* a, const FormArgs* L, int
   if (!a) {
     // rank-1 form only
     if (loadm == dev::LOAD_NONE) fail(DB2_ERR_ARGUMENT, "nothing to assemble");
-    if (load_over_patches(P) && launch_patch_load(P, p, loadm, stream)) return;
+    if (load_over_patches(P) && !writes_coefficients(P, p) && launch_patch_load(P, p, loadm, stream)) return;
     pack_vertex_records(P, nullptr, loadm == dev::LOAD_P1 ? p.f : nullptr, stream);
     // the node rows of the pattern's row range (all of them by default)
     const int64_t n0 = P.row_begin, nr = (P.row_end < 0 ? V.nnodes : P.row_end) - n0;
@@ -228,6 +239,7 @@ void launch_assemble(const Pattern& P, const FormArgs* a, const FormArgs* L, int
   if (a->f.kind == DB2_FORM_DIFFUSION) {
     if (P.bs != 1) fail(DB2_ERR_UNSUPPORTED, "diffusion form on a vector space");
     const bool kp1 = matrix_coeff(*a, p);
+    cfg.latency = cfg.latency && !writes_coefficients(P, p);
     if (!cfg.latency)
       pack_vertex_records(P, kp1 ? p.kappa : nullptr,
                         (loadm == dev::LOAD_P1 || loadm == dev::LOAD_KP1) ? p.f : nullptr, stream);

@@ -399,7 +399,6 @@ void launch_patch_apply(const Pattern& P, const dev::AsmParams& p, bool elas, bo
   dev::PatchArgs q{};
   static_cast<dev::PatchView&>(q) = patch_view(B, elas ? dev::patch_ctas<dev::FORM_ELAS>() : dev::patch_ctas<dev::FORM_DIFF>());
   q.xw = p.xw;
-  q.kappa = kp1 ? p.kappa : nullptr;
   q.kscale = p.kscale;
   q.mu = p.mu;
   q.lmbda = p.lmbda;
@@ -407,14 +406,18 @@ void launch_patch_apply(const Pattern& P, const dev::AsmParams& p, bool elas, bo
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   CallScratch work(P, stream);
   q.partial = work.take(&PatchPlan::Work::partial, B.npartial * P.bs);
-  // a patch writes its finished nodes while others still read x, and reads it
-  // through the read-only path: an x that shares memory with y is copied first
-  if (x < y + n && y < x + n) {
-    double* c = work.take(&PatchPlan::Work::x, n);
-    cudaMemcpyAsync(c, x, size_t(n) * sizeof(double), cudaMemcpyDeviceToDevice, s);
-    check_cuda("copy of x");
-    x = c;
-  }
+  // a patch writes its finished nodes while others still read x and kappa, and
+  // reads them through the read-only path: one that shares memory with y is
+  // copied first
+  auto apart = [&](const double* v, int64_t m, DeviceBuffer PatchPlan::Work::*kept) {
+    if (!overlap(y, n, v, m)) return v;
+    double* c = work.take(kept, m);
+    cudaMemcpyAsync(c, v, size_t(m) * sizeof(double), cudaMemcpyDeviceToDevice, s);
+    check_cuda("copy of an input of the action");
+    return static_cast<const double*>(c);
+  };
+  x = apart(x, n, &PatchPlan::Work::x);
+  if (kp1) q.kappa = apart(p.kappa, P.V->mesh->nv, &PatchPlan::Work::kappa);
   q.x = x;
   q.y = y;
   q.nnodes = p.nnodes;

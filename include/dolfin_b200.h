@@ -239,7 +239,9 @@ int db2_pattern_row_block_csr_host(db2_pattern P, int32_t* rowptr, int32_t* cols
    aligned like every double array here; other pointers are refused with
    DB2_ERR_ARGUMENT).  w is
    the device P1 coefficient (kappa) when a.coeff is P1/P1_SCALED.
-   add_values as AssemblerBase.h:46 (accumulate into vals). */
+   add_values as AssemblerBase.h:46 (accumulate into vals).  The outputs of
+   the assembly entry points and of db2_apply may share memory with kappa, and
+   with a load's f on triangles; on tetrahedra f must lie apart. */
 int db2_assemble_matrix(db2_pattern P, const db2_form* a, const double* w, int precision,
                         double* vals, int add_values, void* stream);
 /* Assembler::assemble(b, L) for a linear form: b[N] (device). */
