@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <array>
 #include <cstdint>
+#include <exception>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -21,7 +22,9 @@ struct Error {
 };
 [[noreturn]] void fail(int code, const char* fmt, ...);
 
-// Run f(begin, end) over [0, n) on up to hardware_concurrency threads.
+// Run f(begin, end) over [0, n) on up to hardware_concurrency threads.  The
+// first exception of a part is thrown again once all parts are done; a part for
+// which no thread can be started runs on the caller's.
 template <typename F>
 void parallel_for(int64_t n, F&& f, int64_t min_chunk = 4096) {
   int nt = (int)std::max(1u, std::thread::hardware_concurrency());
@@ -30,14 +33,30 @@ void parallel_for(int64_t n, F&& f, int64_t min_chunk = 4096) {
     f((int64_t)0, n);
     return;
   }
+  std::exception_ptr error;
+  std::mutex lock;
+  auto part = [&](int64_t b, int64_t e) {
+    try {
+      f(b, e);
+    } catch (...) {
+      std::lock_guard<std::mutex> guard(lock);
+      if (!error) error = std::current_exception();
+    }
+  };
   std::vector<std::thread> th;
+  th.reserve(size_t(nt));
   const int64_t chunk = (n + nt - 1) / nt;
   for (int t = 0; t < nt; ++t) {
     const int64_t b = t * chunk, e = std::min(n, b + chunk);
     if (b >= e) break;
-    th.emplace_back([&f, b, e] { f(b, e); });
+    try {
+      th.emplace_back(part, b, e);
+    } catch (const std::exception&) {  // (system_error, or no memory for its state)
+      part(b, e);
+    }
   }
   for (auto& t : th) t.join();
+  if (error) std::rethrow_exception(error);
 }
 
 // Whether n doubles at a and m doubles at b share memory (NULL: none).
