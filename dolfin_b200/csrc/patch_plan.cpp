@@ -19,6 +19,11 @@ struct Bisector {
   const std::vector<uint32_t>& cell0;  // first cell (by first vertex) of each vertex
   int max_cells;
 
+  // (zero for a coordinate that is no number or infinite: the order below must be one)
+  double coord(int64_t v, int r) const {
+    const double x = m.x[v * m.tdim + r];
+    return std::isfinite(x) ? x : 0.0;
+  }
   int64_t cells_of(const uint32_t* v, int64_t n) const {
     int64_t c = 0;
     for (int64_t i = 0; i < n; ++i) c += cell0[v[i] + 1] - cell0[v[i]];
@@ -29,17 +34,17 @@ struct Bisector {
   int64_t split(uint32_t* v, int64_t n) const {
     const int D = m.tdim;
     double lo[3], hi[3];
-    for (int r = 0; r < D; ++r) lo[r] = hi[r] = m.x[int64_t(v[0]) * D + r];
+    for (int r = 0; r < D; ++r) lo[r] = hi[r] = coord(v[0], r);
     for (int64_t i = 1; i < n; ++i)
       for (int r = 0; r < D; ++r) {
-        const double x = m.x[int64_t(v[i]) * D + r];
+        const double x = coord(v[i], r);
         lo[r] = std::min(lo[r], x);
         hi[r] = std::max(hi[r], x);
       }
     int axis = 0;
     for (int r = 1; r < D; ++r)
       if (hi[r] - lo[r] > hi[axis] - lo[axis]) axis = r;
-    auto key = [&](uint32_t a) { return m.x[int64_t(a) * D + axis]; };
+    auto key = [&](uint32_t a) { return coord(a, axis); };
     auto less = [&](uint32_t a, uint32_t b) {
       const double p = key(a), q = key(b);
       return p < q || (!(q < p) && a < b);

@@ -1,0 +1,57 @@
+"""Cell patches on the host (csrc/patch_plan.cpp), by a program linked to the
+engine that stands in for its device calls: meshes with coordinates that are no
+numbers."""
+import os
+import shutil
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+CSRC, LIB = os.path.join(ROOT, "dolfin_b200", "csrc"), os.path.join(ROOT, "dolfin_b200", "_lib")
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+PRELUDE = r"""
+#include <cmath>
+#include <cstdio>
+#include <limits>
+#include <new>
+#include "internal.h"
+using namespace db2;
+#define CHECK(c) do { if (!(c)) { std::printf("line %d: %s\n", __LINE__, #c); return 1; } } while (0)
+"""
+
+
+def _run(tmp_path, body):
+    cxx = shutil.which(os.environ.get("CXX", "g++"))
+    if cxx is None or not os.path.exists(os.path.join(LIB, "libdolfin_b200.so")):
+        pytest.skip("needs a C++ compiler and the built engine")
+    src, exe = tmp_path / "main.cpp", tmp_path / "main"
+    src.write_text(PRELUDE + body)
+    cuda = os.path.join(CUDA, "lib64")
+    subprocess.run([cxx, "-std=c++17", "-O1", "-pthread", "-rdynamic", "-I", CSRC, str(src), "-o", str(exe), "-L", LIB,
+                    "-ldolfin_b200", f"-Wl,-rpath,{LIB}", "-L", cuda, "-lcudart", f"-Wl,-rpath,{cuda}"], check=True)
+    done = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert done.returncode == 0, done.stdout + done.stderr
+
+
+def test_coordinates_that_are_no_numbers(tmp_path):
+    """The patches are those of the mesh with zeros in their place."""
+    _run(tmp_path, r"""
+int main() {
+  const double bad[] = {std::nan(""), std::numeric_limits<double>::infinity(), -std::numeric_limits<double>::infinity()};
+  for (int dim : {2, 3}) {
+    std::unique_ptr<PatchPlan> plan[2];
+    for (int zero : {0, 1}) {
+      auto m = dim == 3 ? make_unit_cube(14, 12, 13) : make_unit_square(60, 50, 0);
+      for (int64_t i = 0; i < m->nv; i += 37)
+        for (int r = 0; r < dim; ++r) m->x[i * dim + r] = zero ? 0.0 : bad[(i / 37 + r) % 3];
+      auto P = make_pattern(make_space(m, 2, 1), false);
+      plan[zero] = make_patches(*P, 64);
+    }
+    CHECK(plan[0]->npatches == plan[1]->npatches && plan[0]->npartial == plan[1]->npartial);
+    CHECK(plan[0]->nodes == plan[1]->nodes && plan[0]->conn == plan[1]->conn && plan[0]->chunks == plan[1]->chunks);
+  }
+  return 0;
+}
+""")
