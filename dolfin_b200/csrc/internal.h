@@ -308,6 +308,7 @@ struct Pattern {
   const FacetPlan& facet_plan();     // built and uploaded on first use
   mutable std::mutex patches_lock;
   mutable std::unique_ptr<PatchPlan> patches;  // built on first use (patch_plan)
+  mutable bool patches_refused = false;        // by patch_plan_for_loads
 };
 
 // Relabelling of a cell so that local node `li` becomes canonical: for a
@@ -343,6 +344,10 @@ void build_facet_plan(Pattern& P);
 std::unique_ptr<PatchPlan> make_patches(const Pattern& P, int max_cells);
 // The pattern's patches, built and uploaded on first use.
 const PatchPlan& patch_plan(const Pattern& P);
+// The same for load vectors, which the row kernel can do as well: null where
+// there was no memory for the patches or the pattern is beyond their limits.
+// Then it stays so: no other attempt at every call, and the same sums in all.
+const PatchPlan* patch_plan_for_loads(const Pattern& P);
 // Work space of one call over the pattern's patches, from before its first
 // launch until behind its last.  Calls on one stream and pattern take turns.
 class CallScratch {

@@ -158,20 +158,21 @@ bool launch_patch_load(const Pattern& P, const dev::AsmParams& p, int loadm, voi
   // A graph's replays may overlap one another and later calls, so a captured
   // call would need partial sums of its own for the graph's life.
   if (stream_is_capturing(stream)) return false;
+  const PatchPlan* plan = patch_plan_for_loads(P);
+  if (!plan) return false;
+  const PatchPlan& B = *plan;
   std::optional<CallScratch> work;
   double* partial = nullptr;
   int64_t npatches = 0;
   const uint32_t* list = nullptr;
   try {
-    const PatchPlan& B = patch_plan(P);
     npatches = patches_of_rows(P, &list);
     work.emplace(P, stream);
     partial = work->take(&PatchPlan::Work::partial, B.npartial);
-  } catch (const Error&) {  // no room for the plan or the partial sums
-    cudaGetLastError();
-    return false;
+  } catch (const Error& e) {
+    if (e.code != DB2_ERR_NOMEM) throw;
+    return false;  // no room for the partial sums: this call by rows
   }
-  const PatchPlan& B = *P.patches;
   const int D = P.V->mesh->tdim, deg = P.V->degree;
   dev::PatchLoadArgs q{};
   static_cast<dev::PatchView&>(q) = patch_view(B, 5);

@@ -372,6 +372,22 @@ const PatchPlan& patch_plan(const Pattern& P) {
   return *P.patches;
 }
 
+const PatchPlan* patch_plan_for_loads(const Pattern& P) {
+  {
+    std::lock_guard<std::mutex> guard(P.patches_lock);
+    if (P.patches_refused) return nullptr;
+  }
+  try {
+    return &patch_plan(P);
+  } catch (const Error& e) {
+    if (e.code != DB2_ERR_NOMEM && e.code != DB2_ERR_UNSUPPORTED) throw;
+  } catch (const std::bad_alloc&) {
+  }
+  std::lock_guard<std::mutex> guard(P.patches_lock);
+  P.patches_refused = true;
+  return nullptr;
+}
+
 // Work space that stays with a stream costs a call nothing; from the pool it
 // put 1.4 to 1.9 us between the kernels of one call and the next (B200:
 // elasticity P2 action n=48 84.5 -> 85.8 us, FP32 P2 63x70x57 78.3 -> 80.2).

@@ -1,6 +1,6 @@
 """Cell patches on the host (csrc/patch_plan.cpp), by a program linked to the
 engine that stands in for its device calls: meshes with coordinates that are no
-numbers."""
+numbers, and plans that there is no memory for."""
 import os
 import shutil
 import subprocess
@@ -52,6 +52,54 @@ int main() {
     CHECK(plan[0]->npatches == plan[1]->npatches && plan[0]->npartial == plan[1]->npartial);
     CHECK(plan[0]->nodes == plan[1]->nodes && plan[0]->conn == plan[1]->conn && plan[0]->chunks == plan[1]->chunks);
   }
+  return 0;
+}
+""")
+
+
+# uploads that succeed, fail for want of memory, or fail otherwise
+UPLOADS = r"""
+static int uploads = 0, failure = DB2_OK;
+namespace db2 {
+PlanUpload::PlanUpload() {}
+PlanUpload::~PlanUpload() {}
+void PlanUpload::put(DeviceBuffer&, const void*, size_t) {
+  ++uploads;
+  if (failure != DB2_OK) fail(failure, "stand-in");
+}
+}  // namespace db2
+static std::shared_ptr<Pattern> pattern() { return make_pattern(make_space(make_unit_cube(6, 5, 4), 2, 1), false); }
+"""
+
+
+def test_patches_that_cannot_be_built(tmp_path):
+    """A load vector's plan that failed for want of memory, or lies beyond the
+    plan's limits, is not tried again; another failure is an error each time;
+    an action tries, and fails, each time."""
+    _run(tmp_path, UPLOADS + r"""
+int main() {
+  for (int code : {DB2_ERR_NOMEM, DB2_ERR_UNSUPPORTED}) {
+    auto P = pattern();
+    failure = code;
+    uploads = 0;
+    CHECK(patch_plan_for_loads(*P) == nullptr && uploads == 1);
+    CHECK(patch_plan_for_loads(*P) == nullptr && uploads == 1);
+    int caught = 0;
+    try { patch_plan(*P); } catch (const Error& e) { caught = e.code; }
+    CHECK(caught == code && uploads == 2);
+    failure = DB2_OK;
+    patch_plan(*P);
+    CHECK(patch_plan_for_loads(*P) == nullptr);
+  }
+  auto P = pattern();
+  failure = DB2_ERR_CUDA;
+  for (int i = 0; i < 2; ++i) {
+    int caught = 0;
+    try { patch_plan_for_loads(*P); } catch (const Error& e) { caught = e.code; }
+    CHECK(caught == DB2_ERR_CUDA);
+  }
+  failure = DB2_OK;
+  CHECK(patch_plan_for_loads(*P) == &patch_plan(*P));
   return 0;
 }
 """)
