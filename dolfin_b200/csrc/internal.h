@@ -228,7 +228,7 @@ struct PatchPlan {
   // per cell: 8 x its local nodes (byte offsets of doubles), padded to 8 bytes
   std::vector<uint16_t> conn;
   std::vector<uint8_t> chunks;   // per patch: destinations (32 a group), groups, codes
-  std::vector<uint32_t> shared;  // nodes with partial sums
+  std::vector<uint32_t> shared;  // nodes with partial sums, ascending
   std::vector<uint32_t> shared_ptr;  // their partial slots, in patch order
   DeviceBuffer d_hdr, d_conn, d_nodes, d_chunks, d_shared, d_shared_ptr;
   // Work space of calls (CallScratch): partial sums, and copies of inputs that
@@ -247,9 +247,17 @@ struct PatchPlan {
   StreamScratch scratch;
   // per patch: its vertex nodes lie in [b[0], b[1]], its edge nodes in [b[2], b[3]]
   std::vector<std::array<uint32_t, 4>> bounds;
-  // patches meeting the row range they were listed for
-  mutable int64_t list_begin = -1, list_end = -1, list_size = 0;
-  mutable DeviceBuffer d_list;
+  // What a load vector over the node rows [begin, end) takes: the patches that
+  // may hold one of them (on the device), the shared nodes among them and
+  // their partial slots, and whether there are vertex and edge nodes.
+  struct RowSet {
+    int64_t begin = 0, end = 0, npatches = 0;
+    DeviceBuffer list;
+    uint32_t shared0 = 0, shared1 = 0, slot0 = 0, slot1 = 0;
+    bool verts = false, edges = false;
+  };
+  static constexpr size_t kRowSets = 16;  // kept; the oldest goes first
+  mutable std::vector<std::shared_ptr<const RowSet>> row_sets;
   static constexpr uint32_t pad16(uint32_t n) { return (n + 15u) & ~15u; }
 };
 
@@ -364,9 +372,8 @@ class CallScratch {
   std::unique_lock<std::mutex> busy_;
   std::vector<void*> taken_;
 };
-// How many patches the pattern's row range needs, and their numbers on the
-// device (null: all of them).  After patch_plan(P).
-int64_t patches_of_rows(const Pattern& P, const uint32_t** list);
+// The row set of the pattern's row range, or null: all rows.  After patch_plan(P).
+std::shared_ptr<const PatchPlan::RowSet> row_set(const Pattern& P);
 // Re-cut the tiles of an existing plan (autotuning), re-uploading d_tiles.
 void retile(Pattern& P, int tile_threads, int seg_cap_bytes);
 // Tiles of a pattern for a launch shape (pure; does not modify P).

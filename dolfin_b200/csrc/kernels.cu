@@ -161,9 +161,10 @@ static bool latency_bound(const Pattern& P, bool fp32) {
 // n=72 227 -> 93, n=96 430 -> 193; P1 tets n=20 (192,000) 15 -> 20, n=40 17 ->
 // 15, n=60 55 -> 31; P2 triangles n=200 (480,000) 14 -> 15, 500x300 (1.8 M) 22.4
 // -> 21.8.
-// One eighth of P2 n=96's rows (set_row_range): 49 -> 43-56; the eighth
-// that holds the vertices, which meet every patch, 149 -> 187, kept so that a share
-// of the rows equals the whole vector's bit for bit.
+// By the pattern's size, not the row range's, so that a range's rows equal the
+// whole vector's bit for bit; one eighth of P2 n=96's rows (set_row_range) takes
+// 29-43 us against 49-60 by rows, the eighth that holds the vertices, which
+// meet every patch, 145 against 150 (constant f) and 178 (P1 f).
 static bool load_over_patches(const Pattern& P) {
   return int64_t(P.inc.size()) >= (P.V->mesh->tdim == 3 ? 200000 : 1500000);
 }

@@ -16,8 +16,11 @@ namespace dev {
 
 struct PatchLoadArgs : PatchView {
   int bs;
-  uint32_t row_begin, row_end;  // node rows to assemble
-  const uint32_t* list;         // the patches that may hold some of them; null: all
+  // of a row range (RANGED): the patches that may hold its rows, the rows, their
+  // partial slots, and which kinds of nodes are among them
+  const uint32_t* list;
+  uint32_t row_begin, row_end, slot_begin, slot_end;
+  bool verts, edges;
 };
 
 template <int D, int P, int LOADM, int LI>
@@ -38,10 +41,11 @@ __device__ __forceinline__ void stage_load(const AsmParams& p, double vol, const
     ys[LI * stride] = load_row<D, P, LOADM>(p, G, LI <= D, 0, fc, unused);
   }
 }
-template <int D, int P, int LOADM, int... LI>
-__device__ __forceinline__ void stage_loads(const AsmParams& p, double vol, const double (&fv)[D + 1], double* ys,
-                                            int stride, std::integer_sequence<int, LI...>) {
-  (stage_load<D, P, LOADM, LI>(p, vol, fv, ys, stride), ...);
+template <int D, int P, int LOADM, bool RANGED, int... LI>
+__device__ __forceinline__ void stage_loads(const AsmParams& p, const PatchLoadArgs& q, double vol,
+                                            const double (&fv)[D + 1], double* ys, std::integer_sequence<int, LI...>) {
+  auto wanted = [&](bool vertex) { return !RANGED || (vertex ? q.verts : q.edges); };
+  ((wanted(LI <= D) ? stage_load<D, P, LOADM, LI>(p, vol, fv, ys, q.stride) : void()), ...);
 }
 
 __device__ __forceinline__ void put_load(const AsmParams& p, int c, int64_t node, double v) {
@@ -50,7 +54,9 @@ __device__ __forceinline__ void put_load(const AsmParams& p, int c, int64_t node
 }
 
 constexpr int kLoadThreads = 128;
-template <int D, int P, int LOADM>
+// RANGED, the rows of a row range alone: what no row of it takes is neither
+// staged nor summed.
+template <int D, int P, int LOADM, bool RANGED>
 __global__ void __launch_bounds__(kLoadThreads, 5) k_patch_load(const AsmParams p, const PatchLoadArgs q) {
   constexpr int NB = D + 1, K = El<D, P>::K, T = kLoadThreads;
   extern __shared__ __align__(16) unsigned char smem[];
@@ -59,7 +65,7 @@ __global__ void __launch_bounds__(kLoadThreads, 5) k_patch_load(const AsmParams 
   double* vs = reinterpret_cast<double*>(smem);
   double* ys = vs + 4 * q.nv;
   unsigned char* jobs = smem + PatchPlan::pad16(uint32_t((4 * q.nv + K * q.stride + 1) * 8));
-  auto patch = [&](uint32_t i) { return q.list ? __ldg(q.list + i) : i; };
+  auto patch = [&](uint32_t i) { return RANGED ? __ldg(q.list + i) : i; };
   const PatchHdr h = patch_header(q.hdr, patch(blockIdx.x));
   const uint32_t later = blockIdx.x + q.ahead;
   PatchHdr hn{};
@@ -93,23 +99,33 @@ __global__ void __launch_bounds__(kLoadThreads, 5) k_patch_load(const AsmParams 
     if (c + T < h.ncells) cn.load(q, h, c + T);
     Geometry<D> G;
     geometry(x, G);
-    stage_loads<D, P, LOADM>(p, G.vol, fv, ys + c, q.stride, std::make_integer_sequence<int, K>{});
+    stage_loads<D, P, LOADM, RANGED>(p, q, G.vol, fv, ys + c, std::make_integer_sequence<int, K>{});
   }
   __syncthreads();
   const PatchJobs J = patch_jobs(h, jobs);
   const int lane = threadIdx.x & 31;
   for (int g = threadIdx.x >> 5; g < h.ngroups; g += T / 32) {
     const PatchGroup gr = J.groups[g];
+    uint32_t d = 0;
+    bool mine = lane < gr.live;
+    if (RANGED) {
+      if (mine) {
+        d = J.dest[32 * g + lane];
+        const uint32_t t = d & ~kPatchPartial;
+        mine = d & kPatchPartial ? t >= q.slot_begin && t < q.slot_end : t >= q.row_begin && t < q.row_end;
+      }
+      if (!__any_sync(0xffffffffu, mine)) continue;
+    }
     const uint16_t* code = J.codes + gr.code0 + lane;
     double s = 0.0;
 #pragma unroll 4
     for (int t = 0; t < gr.width; ++t)
       s += *reinterpret_cast<const double*>(reinterpret_cast<const char*>(ys) + code[32 * t]);
-    if (lane < gr.live) {
-      const uint32_t d = J.dest[32 * g + lane];
+    if (mine) {
+      if (!RANGED) d = J.dest[32 * g + lane];
       if (d & kPatchPartial) {
         q.partial[d & ~kPatchPartial] = s;
-      } else if (d >= q.row_begin && d < q.row_end) {
+      } else {
         for (int c = 0; c < q.bs; ++c) put_load(p, c, d, LOADM == LOAD_CONST ? s * p.fc[c] : s);
       }
     }
@@ -123,17 +139,16 @@ __global__ void __launch_bounds__(256) k_patch_load_sum(const AsmParams p, const
   const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= n) return;
   const uint32_t node = __ldg(shared + i);
-  if (node < q.row_begin || node >= q.row_end) return;
   double s = 0.0;
   const uint32_t s1 = __ldg(ptr + i + 1);
   for (uint32_t t = __ldg(ptr + i); t < s1; ++t) s += __ldg(q.partial + t);
   for (int c = 0; c < q.bs; ++c) put_load(p, c, node, LOADM == LOAD_CONST ? s * p.fc[c] : s);
 }
 
-template <int D, int P, int LOADM>
-void run_patch_load(const PatchPlan& B, int64_t npatches, const AsmParams& p, const PatchLoadArgs& q, cudaStream_t s) {
+template <int D, int P, int LOADM, bool RANGED>
+void launch_patches(const PatchPlan& B, int64_t npatches, const AsmParams& p, const PatchLoadArgs& q, cudaStream_t s) {
   constexpr int K = El<D, P>::K;
-  auto kern = k_patch_load<D, P, LOADM>;
+  auto kern = k_patch_load<D, P, LOADM, RANGED>;
   static unsigned long long configured = 0;
   allow_dynamic_smem(kern, configured);
   const size_t smem =
@@ -143,9 +158,18 @@ void run_patch_load(const PatchPlan& B, int64_t npatches, const AsmParams& p, co
     count_launch();
     check_cuda("patch load launch");
   }
-  if (B.nshared > 0) {
-    k_patch_load_sum<LOADM><<<unsigned((B.nshared + 255) / 256), 256, 0, s>>>(
-        p, q, B.d_shared.as<uint32_t>(), B.d_shared_ptr.as<uint32_t>(), B.nshared);
+}
+
+template <int D, int P, int LOADM>
+void run_patch_load(const PatchPlan& B, const PatchPlan::RowSet* rows, const AsmParams& p, const PatchLoadArgs& q,
+                    cudaStream_t s) {
+  if (rows) launch_patches<D, P, LOADM, true>(B, rows->npatches, p, q, s);
+  else launch_patches<D, P, LOADM, false>(B, B.npatches, p, q, s);
+  const uint32_t s0 = rows ? rows->shared0 : 0;
+  const int64_t n = rows ? rows->shared1 - s0 : B.nshared;
+  if (n > 0) {
+    k_patch_load_sum<LOADM><<<unsigned((n + 255) / 256), 256, 0, s>>>(p, q, B.d_shared.as<uint32_t>() + s0,
+                                                                      B.d_shared_ptr.as<uint32_t>() + s0, n);
     count_launch();
     check_cuda("patch load sum launch");
   }
@@ -163,10 +187,9 @@ bool launch_patch_load(const Pattern& P, const dev::AsmParams& p, int loadm, voi
   const PatchPlan& B = *plan;
   std::optional<CallScratch> work;
   double* partial = nullptr;
-  int64_t npatches = 0;
-  const uint32_t* list = nullptr;
+  std::shared_ptr<const PatchPlan::RowSet> rows;
   try {
-    npatches = patches_of_rows(P, &list);
+    rows = row_set(P);
     work.emplace(P, stream);
     partial = work->take(&PatchPlan::Work::partial, B.npartial);
   } catch (const Error& e) {
@@ -178,13 +201,19 @@ bool launch_patch_load(const Pattern& P, const dev::AsmParams& p, int loadm, voi
   static_cast<dev::PatchView&>(q) = patch_view(B, 5);
   q.partial = partial;
   q.bs = P.bs;
-  q.row_begin = uint32_t(P.row_begin);
-  q.row_end = uint32_t(P.row_end < 0 ? P.V->nnodes : P.row_end);
-  q.list = list;
+  if (rows) {
+    q.list = rows->list.as<uint32_t>();
+    q.row_begin = uint32_t(rows->begin);
+    q.row_end = uint32_t(rows->end);
+    q.slot_begin = rows->slot0;
+    q.slot_end = rows->slot1;
+    q.verts = rows->verts;
+    q.edges = rows->edges;
+  }
 #define DB2_PL(D_, P_)                                                                           \
   if (D == D_ && deg == P_) {                                                                    \
-    if (loadm == dev::LOAD_CONST) dev::run_patch_load<D_, P_, dev::LOAD_CONST>(B, npatches, p, q, s);      \
-    else dev::run_patch_load<D_, P_, dev::LOAD_P1>(B, npatches, p, q, s);                                  \
+    if (loadm == dev::LOAD_CONST) dev::run_patch_load<D_, P_, dev::LOAD_CONST>(B, rows.get(), p, q, s); \
+    else dev::run_patch_load<D_, P_, dev::LOAD_P1>(B, rows.get(), p, q, s);                     \
     return true;                                                                                 \
   }
   DB2_PL(3, 1) DB2_PL(3, 2) DB2_PL(2, 1) DB2_PL(2, 2)

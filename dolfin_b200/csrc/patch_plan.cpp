@@ -365,8 +365,9 @@ const PatchPlan& patch_plan(const Pattern& P) {
     up(B->d_conn, B->conn);
     up(B->d_nodes, B->nodes);
     up(B->d_chunks, B->chunks);
-    up(B->d_shared, B->shared);
-    up(B->d_shared_ptr, B->shared_ptr);
+    // (these two stay on the host too, for the row sets)
+    if (B->nshared > 0) U.put(B->d_shared, B->shared.data(), B->shared.size() * sizeof(uint32_t));
+    U.put(B->d_shared_ptr, B->shared_ptr.data(), B->shared_ptr.size() * sizeof(uint32_t));
     P.patches = std::move(B);
   }
   return *P.patches;
@@ -430,27 +431,36 @@ double* CallScratch::take(DeviceBuffer PatchPlan::Work::*which, int64_t n) {
   return static_cast<double*>(p);
 }
 
-int64_t patches_of_rows(const Pattern& P, const uint32_t** list) {
+std::shared_ptr<const PatchPlan::RowSet> row_set(const Pattern& P) {
   const PatchPlan& B = *P.patches;
   const int64_t r0 = P.row_begin, r1 = P.row_end < 0 ? P.V->nnodes : P.row_end;
-  *list = nullptr;
-  if (r0 == 0 && r1 == P.V->nnodes) return B.npatches;
-  if (r0 >= r1) return 0;
+  if (r0 == 0 && r1 == P.V->nnodes) return nullptr;
   std::lock_guard<std::mutex> guard(P.patches_lock);
-  if (B.list_begin != r0 || B.list_end != r1) {
-    std::vector<uint32_t> ids;
-    auto meets = [&](uint32_t a, uint32_t b) { return a <= b && a < r1 && b >= r0; };
-    for (size_t i = 0; i < B.bounds.size(); ++i)
-      if (meets(B.bounds[i][0], B.bounds[i][1]) || meets(B.bounds[i][2], B.bounds[i][3])) ids.push_back(uint32_t(i));
-    B.list_begin = -1;
-    PlanUpload U;
-    U.put(B.d_list, ids.data(), ids.size() * sizeof(uint32_t));
-    B.list_size = int64_t(ids.size());
-    B.list_begin = r0;
-    B.list_end = r1;
-  }
-  *list = B.d_list.as<uint32_t>();
-  return B.list_size;
+  for (const auto& s : B.row_sets)
+    if (s->begin == r0 && s->end == r1) return s;
+  auto S = std::make_shared<PatchPlan::RowSet>();
+  S->begin = r0;
+  S->end = r1;
+  S->verts = r0 < r1 && r0 < P.V->mesh->nv;
+  S->edges = r0 < r1 && r1 > P.V->mesh->nv;
+  auto first = [&](int64_t row) {
+    return uint32_t(std::lower_bound(B.shared.begin(), B.shared.end(), uint32_t(row)) - B.shared.begin());
+  };
+  S->shared0 = first(r0);
+  S->shared1 = std::max(S->shared0, first(r1));
+  S->slot0 = B.shared_ptr[S->shared0];
+  S->slot1 = B.shared_ptr[S->shared1];
+  std::vector<uint32_t> ids;
+  auto meets = [&](uint32_t a, uint32_t b) { return r0 < r1 && a <= b && a < r1 && b >= r0; };
+  for (size_t i = 0; i < B.bounds.size(); ++i)
+    if (meets(B.bounds[i][0], B.bounds[i][1]) || meets(B.bounds[i][2], B.bounds[i][3])) ids.push_back(uint32_t(i));
+  S->npatches = int64_t(ids.size());
+  PlanUpload U;
+  U.put(S->list, ids.data(), ids.size() * sizeof(uint32_t));
+  // (a call in progress on another thread holds the set that goes)
+  if (B.row_sets.size() >= PatchPlan::kRowSets) B.row_sets.erase(B.row_sets.begin());
+  B.row_sets.push_back(S);
+  return S;
 }
 
 }  // namespace db2

@@ -1,6 +1,6 @@
 """Cell patches on the host (csrc/patch_plan.cpp), by a program linked to the
 engine that stands in for its device calls: meshes with coordinates that are no
-numbers, and plans that there is no memory for."""
+numbers, plans that there is no memory for, and the patches of row ranges."""
 import os
 import shutil
 import subprocess
@@ -60,11 +60,13 @@ int main() {
 # uploads that succeed, fail for want of memory, or fail otherwise
 UPLOADS = r"""
 static int uploads = 0, failure = DB2_OK;
+static std::vector<uint32_t> last;  // what was uploaded last
 namespace db2 {
 PlanUpload::PlanUpload() {}
 PlanUpload::~PlanUpload() {}
-void PlanUpload::put(DeviceBuffer&, const void*, size_t) {
+void PlanUpload::put(DeviceBuffer&, const void* host, size_t n) {
   ++uploads;
+  last.assign(static_cast<const uint32_t*>(host), static_cast<const uint32_t*>(host) + n / 4);
   if (failure != DB2_OK) fail(failure, "stand-in");
 }
 }  // namespace db2
@@ -100,6 +102,56 @@ int main() {
   }
   failure = DB2_OK;
   CHECK(patch_plan_for_loads(*P) == &patch_plan(*P));
+  return 0;
+}
+""")
+
+
+def test_row_sets(tmp_path):
+    """A row range's patches, shared nodes and partial slots are those that its
+    rows meet, by the plan; a range that comes back (ranges of several ranks in
+    turn) is not listed again."""
+    _run(tmp_path, UPLOADS + r"""
+int main() {
+  auto P = pattern();
+  patch_plan(*P);
+  auto B = make_patches(*P, 64);  // what patch_plan builds for a mesh of 720 cells
+  const int64_t nn = P->V->nnodes, nv = P->V->mesh->nv;
+  CHECK(row_set(*P) == nullptr && B->npatches > 8);
+  const int64_t cuts[][2] = {{0, 0}, {0, nv}, {nv, nn}, {3, 40}, {nv - 5, nv + 7}, {nn - 1, nn}, {0, nn - 1}, {nn, nn}};
+  for (auto& c : cuts) {
+    P->row_begin = c[0];
+    P->row_end = c[1] == nn ? -1 : c[1];
+    last.clear();
+    auto S = row_set(*P);
+    auto in = [&](uint32_t n) { return n >= c[0] && n < c[1]; };
+    CHECK(S && S->npatches == int64_t(last.size()));
+    size_t at = 0;
+    for (int64_t i = 0; i < B->npatches; ++i) {
+      bool meets = false;
+      for (int j = 0; j < B->hdr[i].nnodes; ++j) meets |= in(B->nodes[B->hdr[i].node0 + j]);
+      const bool listed = at < last.size() && last[at] == i;
+      CHECK(listed || !meets);
+      at += listed;
+    }
+    CHECK(at == last.size());
+    for (size_t i = 0; i < B->shared.size(); ++i) CHECK(in(B->shared[i]) == (i >= S->shared0 && i < S->shared1));
+    CHECK(S->slot0 == B->shared_ptr[S->shared0] && S->slot1 == B->shared_ptr[S->shared1]);
+    CHECK(S->verts == (c[0] < c[1] && c[0] < nv) && S->edges == (c[0] < c[1] && c[1] > nv));
+  }
+  const int before = uploads;
+  for (int turn = 0; turn < 3; ++turn)
+    for (auto& c : cuts) {
+      P->row_begin = c[0];
+      P->row_end = c[1] == nn ? -1 : c[1];
+      CHECK(row_set(*P)->begin == c[0]);
+    }
+  CHECK(uploads == before);
+  for (int64_t i = 1; i < 40; ++i) {  // more than are kept
+    P->row_begin = i;
+    CHECK(row_set(*P)->begin == i);
+  }
+  CHECK(P->patches->row_sets.size() == PatchPlan::kRowSets);
   return 0;
 }
 """)
