@@ -155,18 +155,33 @@ static bool latency_bound(const Pattern& P, bool fp32) {
 }
 
 // Load vectors over cell patches (patch_load.cu: two launches, every cell once)
-// or by the thread-per-row kernel (one launch, in 2D after a packing one).
-// Measured on B200 (us a call, by rows -> over patches): P2 tets n=10 (60,000
-// incidences) 17 -> 18, n=16 (245,760) 18 -> 15, n=34 33 -> 18, n=50 80 -> 38,
-// n=72 227 -> 93, n=96 430 -> 193; P1 tets n=20 (192,000) 15 -> 20, n=40 17 ->
-// 15, n=60 55 -> 31; P2 triangles n=200 (480,000) 14 -> 15, 500x300 (1.8 M) 22.4
-// -> 21.8.
+// or by the thread-per-row kernel (one launch, in 2D with a P1 f after a packing
+// one): the incidences from which the patches are no slower.  A row's work is
+// the cells around it, once for each component; its kernel is short where a
+// cell's load is one number (constant f) and its geometry cheap (triangles, few
+// cells a row in P1).  Measured on B200, us a call in a loop, by rows / over
+// patches, on both sides of each line:
+//   P1 tets  f P1   n=33 (0.86 M) 14.6 / 15.7, n=34 (0.94 M) 16.5 / 15.8
+//            const  n=52 (3.4 M) 20.6 / 23.2, n=56 (4.2 M) 26.7 / 26.7, n=64 49 / 35
+//            vector n=28 (0.53 M) 14.4 / 15.4, n=30 (0.65 M) 16.6 / 15.5
+//   P2 tets  f P1   n=14 (0.16 M) 17.3 / 15.6, n=24 20.6 / 15.6, n=96 531 / 200
+//            const  n=15 (0.20 M) 14.4 / 15.2, n=18 (0.35 M) 16.4 / 15.2, n=96 431 / 201
+//            vector n=10 (60,000) 14.8 / 15.3, n=18 (0.35 M) 18.5 / 15.1
+//   P1 tris  f P1   n=700 (2.9 M) 22.0 / 22.6, n=750 (3.4 M) 24.7 / 24.6, n=850 31 / 26.7
+//            const  n=850 (4.3 M) 20.5 / 26.7, n=1150 (7.9 M) 40 / 58: always by rows
+//            vector n=500 (1.5 M) 14.6 / 15.5, n=550 (1.8 M) 16.5 / 16.3, n=650 21.7 / 18.5
+//   P2 tris  f P1   n=300 (1.1 M) 16.3 / 15.5, n=360 (1.6 M) 18.5 / 16.0, n=500 30.5 / 18.8
+//            const  n=350 (1.5 M) 12.4 / 15.4, n=460 (2.5 M) 18.5 / 18.5, n=500 (3 M) 23.7 / 20.6
+//            vector n=300 (1.1 M) 16.5 / 15.2, n=400 (1.9 M) 26.7 / 16.5
 // By the pattern's size, not the row range's, so that a range's rows equal the
 // whole vector's bit for bit; one eighth of P2 n=96's rows (set_row_range) takes
 // 29-43 us against 49-60 by rows, the eighth that holds the vertices, which
 // meet every patch, 145 against 150 (constant f) and 178 (P1 f).
-static bool load_over_patches(const Pattern& P) {
-  return int64_t(P.inc.size()) >= (P.V->mesh->tdim == 3 ? 200000 : 1500000);
+static bool load_over_patches(const Pattern& P, int loadm) {
+  const int tdim = P.V->mesh->tdim, kind = loadm == dev::LOAD_P1 ? 0 : P.bs == 1 ? 1 : 2;
+  static const int64_t kLine[2][2][3] = {{{3400000, INT64_MAX, 1800000}, {1500000, 2700000, 1500000}},
+                                         {{900000, 4500000, 640000}, {200000, 300000, 200000}}};
+  return int64_t(P.inc.size()) >= kLine[tdim - 2][P.V->degree - 1][kind];
 }
 
 // Whether the call writes over the memory of its kappa or f.  The tile classes
@@ -204,7 +219,7 @@ void launch_assemble(const Pattern& P, const FormArgs* a, const FormArgs* L, int
   if (!a) {
     // rank-1 form only
     if (loadm == dev::LOAD_NONE) fail(DB2_ERR_ARGUMENT, "nothing to assemble");
-    if (load_over_patches(P) && !writes_coefficients(P, p) && launch_patch_load(P, p, loadm, stream)) return;
+    if (load_over_patches(P, loadm) && !writes_coefficients(P, p) && launch_patch_load(P, p, loadm, stream)) return;
     pack_vertex_records(P, nullptr, loadm == dev::LOAD_P1 ? p.f : nullptr, stream);
     // the node rows of the pattern's row range (all of them by default)
     const int64_t n0 = P.row_begin, nr = (P.row_end < 0 ? V.nnodes : P.row_end) - n0;

@@ -295,8 +295,8 @@ int db2_assemble_facets_bc(db2_pattern P, const db2_form* a_ds, const double* wa
    and calling GenericMatrix::mult (dolfin/la/GenericMatrix.h).  Computed
    per cell (element actions, exact integration) and summed per row in a
    fixed order, so repeated calls agree bitwise; x and y may be one array.
-   The first call on a pattern builds its cell patches (plan arrays of 50 to
-   100 bytes a cell on the device, kept by the pattern).  Partial sums,
+   The first call on a pattern builds its cell patches (plan arrays of 20 to
+   75 bytes a cell on the device, kept by the pattern).  Partial sums,
    about one a cell and component, are kept for each of the first eight
    streams that calls come on and come from a stream-ordered pool on others, so
    calls may overlap on several streams and threads; captured calls share one
