@@ -181,12 +181,23 @@ int db2_batch_create(int count, const db2_pattern* patterns, const db2_form* for
     using namespace db2;
     if (count <= 0 || !patterns || !forms || !kappas || !vals || !out)
       fail(DB2_ERR_ARGUMENT, "batch: empty or NULL arguments");
-    // One-warp tiles by default: their barriers couple no warps.  Measured on B200
-    // (us a replay, 64 / 16 / 256 triangle meshes): 92.6 / 12.6 / 341 against 98.4
-    // / 16.5 / 362 with 128 threads and 24 KB, 96.7 / 13.9 / 353 with 64 threads.
-    const int threads = tile_threads > 0 ? tile_threads : 32;
+    // One-warp tiles by default, their barriers couple no warps, with segments of
+    // 7 KB, so that shared memory lets the 32 blocks of an SM in that the
+    // registers do (only P2 tetrahedra have larger ones at one warp); 128 threads
+    // and 24 KB where there are many P2 tetrahedra.  Measured on B200 (us a
+    // replay, one warp with 7 KB / 16 KB / 128 threads, FP64): triangles P2 n=64
+    // x64 61 / 61 / 64, P1 and P2 n=150 x64 193 / 193 / 204; P1 tets n=20 x64 129 /
+    // 129 / 133; P2 tets n=3 x64 28 / 28 / 35, n=8 x4 27 / 29 / 35, n=12 x4 (62,500
+    // nodes) 30 / 31 / 36, n=8 x64 (314,000) 75 / 90 / 74, n=12 x64 (1.0 M) 204 /
+    // 269 / 204 (FP32 165 / 228 / 156), n=20 x16 (1.1 M) 224 / 291 / 220 (FP32 182
+    // / 246 / 168).
+    int64_t p2_tet_nodes = 0;
+    for (int m = 0; m < count; ++m)
+      if (auto P = pattern_of(patterns[m]))
+        if (P->V->mesh->tdim == 3 && P->V->degree == 2) p2_tet_nodes += P->V->nnodes;
+    const int threads = tile_threads > 0 ? tile_threads : p2_tet_nodes >= 300000 ? 128 : 32;
     if (threads % 32 || threads > dev::kMaxTileThreads) fail(DB2_ERR_ARGUMENT, "batch: tile_threads");
-    const int cap = seg_cap_bytes > 0 ? seg_cap_bytes : 16 * 1024;
+    const int cap = seg_cap_bytes > 0 ? seg_cap_bytes : threads > 32 ? 24 * 1024 : 7 * 1024;
     auto* h = new db2_batch_t;
     Batch& B = h->B;
     try {
