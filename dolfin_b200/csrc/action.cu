@@ -26,6 +26,16 @@ __global__ void __launch_bounds__(256) k_apply_gather(const uint32_t* __restrict
   y[node] = acc;
 }
 
+// A cell's incidences are read at once, in wide loads, and kept, and its vertex
+// nodes taken from its vertices; P2 triangles without a load (LATE) read both for
+// each node where they are used -- measured on B200, us a VJP, at once / late:
+// P2 triangles n=700 94.0 / 90.7 (FP32 97.9 / 93.4), with a load 94.8 / 100.7;
+// P1 tets n=64 83 / 93 and 87 / 103, P2 tets n=40 77 / 91 and 84 / 103.
+template <int D, int P, bool LOADK>
+constexpr bool vjp_late() {
+  return D == 2 && P == 2 && !LOADK;
+}
+
 // gA at the columns of a cell's row by its incidence record, and gb.
 template <int D, int P, bool LOADK>
 struct RecordRow {
@@ -38,10 +48,11 @@ struct RecordRow {
   template <int LI>
   __device__ __forceinline__ void get(double (&g)[El<D, P>::K], double& gbi) const {
     constexpr int K = El<D, P>::K;
-    const uint32_t ii = inc[LI];
+    constexpr bool LATE = vjp_late<D, P, LOADK>();
+    const uint32_t ii = LATE ? __ldg(p.cell_inc + size_t(cell) * K + LI) : inc[LI];
     // vertex nodes are numbered as the vertices (natural numbering)
     uint32_t node;
-    if constexpr (LI <= D) node = v[LI];
+    if constexpr (LI <= D && !LATE) node = v[LI];
     else node = __ldg(p.cell_nodes + size_t(cell) * K + LI);
     const double* grow = gA + __ldg(p.node_rowptr + node);
     const Rec<D, P> rr = load_rec<D, P>(p, rec_index<D, P>(p, node, ii - __ldg(p.inc_ptr + node)));
@@ -77,7 +88,8 @@ __global__ void __maxnreg__((vjp_maxnreg<P>())) k_vjp_cells(const AsmParams p, i
   uint32_t inc[E::K];
   {
     const uint32_t* ci = p.cell_inc + size_t(cell) * E::K;
-    if constexpr (E::K % 4 == 0) {
+    if constexpr (vjp_late<D, P, LOADK>()) {
+    } else if constexpr (E::K % 4 == 0) {
 #pragma unroll
       for (int j = 0; j < E::K; j += 4) {
         const uint4 w = __ldg(reinterpret_cast<const uint4*>(ci + j));
@@ -114,7 +126,8 @@ __global__ void __maxnreg__((vjp_maxnreg<P>())) k_vjp_cells(const AsmParams p, i
   // in vertex-incidence order (vertex nodes come first in the node-contiguous
   // incidence array), so that step 2 reads each vertex's terms contiguously
 #pragma unroll
-  for (int a = 0; a < NB; ++a) t[inc[a]] = acc[a];
+  for (int a = 0; a < NB; ++a)
+    t[vjp_late<D, P, LOADK>() ? __ldg(p.cell_inc + size_t(cell) * E::K + a) : inc[a]] = acc[a];
 }
 
 // Adjoint, step 2 (one thread per vertex): dkappa[v] = sum over cells around
