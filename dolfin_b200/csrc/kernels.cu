@@ -144,13 +144,15 @@ static int load_mode(const FormArgs* L, int bs, dev::AsmParams& p) {
 // (1.05 M) 40 -> 36, n=36 (2.8 M) 78 -> 79; P1 tets n=34 (0.94 M) 23 -> 18, n=38
 // (1.3 M) 21 -> 21, n=44 (2.0 M) 31 -> 38; vector P2 elasticity n=12 (0.93 M)
 // 35 -> 25, n=14 (1.5 M) 35 -> 35; P2 triangles n=200 (0.48 M) 21 -> 14, n=300
-// (1.08 M) 29 -> 30.  FP32 rows of P2 tets spill at their register cap in the
-// tile classes: n=34 (2.4 M) 75 -> 60, n=37 (3.0 M) 86 -> 76, elasticity n=14
-// 49 -> 38, n=18 (3.1 M) 70 -> 69.  By the pattern's size, not the row range's,
-// so that a range's rows equal the whole assembly's bit for bit.
+// (1.08 M) 29 -> 30.  P2 tets in FP32 (74 to 80 registers in
+// the tile classes, no spills) gain longer in a loop, a call after which the host
+// waits does not: n=34 (2.4 M) 71 -> 59 and alone 74 -> 73, n=35 (2.6 M) 73 -> 67
+// and 76 -> 81, n=36 78 -> 69 and 80 -> 83; elasticity n=16 (2.2 M) 51 -> 48 and
+// 62 -> 61, n=18 (3.1 M) 67 -> 66 and 78 -> 77.  By the pattern's size, not the row
+// range's, so that a range's rows equal the whole assembly's bit for bit.
 static bool latency_bound(const Pattern& P, bool fp32) {
   const int64_t incidences = int64_t(P.inc.size()) * P.bs * P.bs;
-  const int64_t line = P.V->mesh->tdim == 2 ? 1000000 : fp32 && P.V->degree == 2 ? 3000000 : 1400000;
+  const int64_t line = P.V->mesh->tdim == 2 ? 1000000 : fp32 && P.V->degree == 2 ? 2400000 : 1400000;
   return incidences <= line && P.rec_escapes == 0;
 }
 
