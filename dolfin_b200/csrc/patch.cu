@@ -11,7 +11,10 @@
 // (60 B a cell), x, y and about one partial sum a cell.  Measured on B200, ms
 // per action: vector P2 elasticity n=48 0.245 -> 0.087, P2 tets n=96 0.342 ->
 // 0.230, P1 tets n=80 0.102 -> 0.060; with FP32 actions 63x70x57 0.084 ->
-// 0.079 (its quadrature is unchanged, and issue-bound).
+// 0.079 (its quadrature is unchanged, and issue-bound).  Least is gained where
+// the cell actions were short: P1 triangles with a constant coefficient in FP32
+// take 0.0165 against 0.0142 at n=600, 0.0226 / 0.0257 at n=900, 0.0637 / 0.0618
+// at n=1500, 0.101 / 0.105 at n=2000.
 #include <cuda_runtime.h>
 
 #include "patch.cuh"
@@ -29,7 +32,7 @@ struct PatchArgs : PatchView {
   int64_t nnodes;
 };
 
-// Element action of P2 by exact moments, FP64.  With U_m the gradient of u at
+// Element action of P2 by exact moments.  With U_m the gradient of u at
 // vertex m (grad u is linear), F the flux and M_m = int lambda_m F:
 //   y_v = g_v . (4 M_v - sum_m M_m),   y_(p,q) = 4 (g_p . M_q + g_q . M_p),
 // where for a linear flux (F_m its vertex values) M_m = |T| c2 (sum F + F_m),
@@ -45,64 +48,64 @@ constexpr double moment3() { return D == 3 ? 1.0 / 120 : 1.0 / 60; }
 
 // Gradients of one P2 component at the vertices: U_m = sum_a d_a g_a with
 // d_a = 4 x_(a,m) - x_a (a != m), 3 x_m (a = m).
-template <int D>
-__device__ __forceinline__ void p2_vertex_gradients(const double (&xc)[El<D, 2>::K], const double (&g)[D + 1][D],
-                                                    double (&U)[D + 1][D]) {
+template <int D, typename CT>
+__device__ __forceinline__ void p2_vertex_gradients(const CT (&xc)[El<D, 2>::K], const CT (&g)[D + 1][D],
+                                                    CT (&U)[D + 1][D]) {
 #pragma unroll
   for (int m = 0; m <= D; ++m) {
 #pragma unroll
-    for (int r = 0; r < D; ++r) U[m][r] = 0.0;
+    for (int r = 0; r < D; ++r) U[m][r] = CT(0);
 #pragma unroll
     for (int a = 0; a <= D; ++a) {
-      const double d = a == m ? 3.0 * xc[m] : fma(4.0, xc[D + 1 + cell_edge_of(D, a, m)], -xc[a]);
+      const CT d = a == m ? CT(3) * xc[m] : fma(CT(4), xc[D + 1 + cell_edge_of(D, a, m)], -xc[a]);
 #pragma unroll
       for (int r = 0; r < D; ++r) U[m][r] = fma(d, g[a][r], U[m][r]);
     }
   }
 }
 
-template <int D>
-__device__ __forceinline__ double dotg(const double (&a)[D], const double (&b)[D]) {
-  double s = a[0] * b[0];
+template <int D, typename CT>
+__device__ __forceinline__ CT dotg(const CT (&a)[D], const CT (&b)[D]) {
+  CT s = a[0] * b[0];
 #pragma unroll
   for (int r = 1; r < D; ++r) s = fma(a[r], b[r], s);
   return s;
 }
 
 // P2 test functions against the moments M and t_v = 4 M_v - sum M.
-template <int D>
-__device__ __forceinline__ void p2_test(const double (&M)[D + 1][D], const double (&t)[D + 1][D],
-                                        const double (&g)[D + 1][D], double (&y)[El<D, 2>::K]) {
+template <int D, typename CT>
+__device__ __forceinline__ void p2_test(const CT (&M)[D + 1][D], const CT (&t)[D + 1][D], const CT (&g)[D + 1][D],
+                                        CT (&y)[El<D, 2>::K]) {
 #pragma unroll
-  for (int v = 0; v <= D; ++v) y[v] = dotg<D>(g[v], t[v]);
+  for (int v = 0; v <= D; ++v) y[v] = dotg<D, CT>(g[v], t[v]);
 #pragma unroll
   for (int e = 0; e < El<D, 2>::NE; ++e) {
     const int p = edge_end(D, e, 0), q = edge_end(D, e, 1);
-    double s = dotg<D>(g[p], M[q]);
+    CT s = dotg<D, CT>(g[p], M[q]);
 #pragma unroll
     for (int r = 0; r < D; ++r) s = fma(g[q][r], M[p][r], s);
-    y[D + 1 + e] = 4.0 * s;
+    y[D + 1 + e] = CT(4) * s;
   }
 }
 
 // A linear flux of vertex values F: M_m = S + F_m with S = sum F (times |T|
 // c2), so t_v = 4 F_v - (D - 2) S.
-template <int D>
-__device__ __forceinline__ void p2_test_linear(const double (&F)[D + 1][D], const double (&g)[D + 1][D],
-                                               double (&y)[El<D, 2>::K]) {
-  double M[D + 1][D], t[D + 1][D];
+template <int D, typename CT>
+__device__ __forceinline__ void p2_test_linear(const CT (&F)[D + 1][D], const CT (&g)[D + 1][D],
+                                               CT (&y)[El<D, 2>::K]) {
+  CT M[D + 1][D], t[D + 1][D];
 #pragma unroll
   for (int r = 0; r < D; ++r) {
-    double S = F[0][r];
+    CT S = F[0][r];
 #pragma unroll
     for (int m = 1; m <= D; ++m) S += F[m][r];
 #pragma unroll
     for (int m = 0; m <= D; ++m) {
       M[m][r] = S + F[m][r];
-      t[m][r] = D == 3 ? fma(4.0, F[m][r], -S) : 4.0 * F[m][r];
+      t[m][r] = D == 3 ? fma(CT(4), F[m][r], -S) : CT(4) * F[m][r];
     }
   }
-  p2_test<D>(M, t, g, y);
+  p2_test<D, CT>(M, t, g, y);
 }
 
 // y_K = A_K x_K of one cell, every component.
@@ -117,7 +120,7 @@ __device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&x
   if constexpr (P == 2 && sizeof(CT) == 8) {
     if constexpr (FORM == FORM_DIFF) {
       double U[NB][D];
-      p2_vertex_gradients<D>(xc[0], g, U);
+      p2_vertex_gradients<D, double>(xc[0], g, U);
       const double w = vol * q.kscale * (KP1 ? moment3<D>() : moment2<D>());
       if constexpr (KP1) {
         double M[NB][D], t[NB][D];
@@ -141,13 +144,13 @@ __device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&x
 #pragma unroll
           for (int m = 0; m <= D; ++m) t[m][r] = fma(4.0, M[m][r], -M0);
         }
-        p2_test<D>(M, t, g, y[0]);
+        p2_test<D, double>(M, t, g, y[0]);
       } else {
 #pragma unroll
         for (int m = 0; m <= D; ++m)
 #pragma unroll
           for (int r = 0; r < D; ++r) U[m][r] *= w;
-        p2_test_linear<D>(U, g, y[0]);
+        p2_test_linear<D, double>(U, g, y[0]);
       }
     } else {
       // stress at the vertices: lambda div(u) I + mu (grad u + grad u^T)
@@ -155,7 +158,7 @@ __device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&x
 #pragma unroll
       for (int e = 0; e < D; ++e) {
         double U[NB][D];
-        p2_vertex_gradients<D>(xc[e], g, U);
+        p2_vertex_gradients<D, double>(xc[e], g, U);
 #pragma unroll
         for (int m = 0; m <= D; ++m)
 #pragma unroll
@@ -183,9 +186,24 @@ __device__ __forceinline__ void cell_action(const PatchArgs& q, const double (&x
         for (int m = 0; m <= D; ++m)
 #pragma unroll
           for (int d = 0; d < D; ++d) F[m][d] = sg[m][c][d];
-        p2_test_linear<D>(F, g, y[c]);
+        p2_test_linear<D, double>(F, g, y[c]);
       }
     }
+  } else if constexpr (P == 2 && FORM == FORM_DIFF && !KP1) {
+    // A linear flux, in FP32 up to the factor |T| kappa.  Measured on B200 against
+    // the five-point rule (ms per action): P2 tets n=64 0.070 against 0.086, P2
+    // triangles n=700 0.031 against 0.037; error 5.3e-8 against 8.2e-8 (rms,
+    // random x) and 2.6e-7 against 3.5e-7 (smooth x).
+    CT gc[NB][D], U[NB][D], yc[K];
+#pragma unroll
+    for (int a = 0; a < NB; ++a)
+#pragma unroll
+      for (int r = 0; r < D; ++r) gc[a][r] = CT(g[a][r]);
+    p2_vertex_gradients<D, CT>(xc[0], gc, U);
+    p2_test_linear<D, CT>(U, gc, yc);
+    const double w = vol * q.kscale * moment2<D>();
+#pragma unroll
+    for (int j = 0; j < K; ++j) y[0][j] = w * double(yc[j]);
   } else {
     // quadrature (P1: the centroid), in the contraction type
     using Q = Quad<D, P == 1 ? 1 : (FORM == FORM_ELAS ? 2 : 3)>;
@@ -263,19 +281,26 @@ template <int FORM>
 constexpr int patch_ctas() {
   return FORM == FORM_ELAS ? 4 : 5;
 }
+// Doubles of a staged vertex: its coordinates and kappa, for 16-byte reads (P1
+// triangles n=1000 with a constant coefficient: 0.0328 ms against 0.0349 with
+// four doubles).
+template <int D, bool KP1>
+constexpr int patch_vertex() {
+  return D == 2 && !KP1 ? 2 : 4;
+}
 template <int D, int P, int FORM, bool KP1, typename CT>
 __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_apply(const PatchArgs q) {
   constexpr int NB = D + 1, K = El<D, P>::K, BS = FORM == FORM_ELAS ? D : 1;
-  constexpr int T = kPatchThreads;
+  constexpr int T = kPatchThreads, VS = patch_vertex<D, KP1>();
   extern __shared__ __align__(16) unsigned char smem[];
   // vertex records (x, y, z, kappa), the nodes' x by component (in the
   // contraction type: one conversion a node, not one a cell and node), the
   // staged actions by component and local node (and a zero slot each), the jobs
   double* vs = reinterpret_cast<double*>(smem);
-  CT* xs = reinterpret_cast<CT*>(vs + 4 * q.nv);
+  CT* xs = reinterpret_cast<CT*>(vs + VS * q.nv);
   CT* ys = xs + BS * q.nx;
   const int plane = K * q.stride + 1;
-  unsigned char* jobs = smem + PatchPlan::pad16(uint32_t(32 * q.nv + BS * (q.nx + plane) * int(sizeof(CT))));
+  unsigned char* jobs = smem + PatchPlan::pad16(uint32_t(8 * VS * q.nv + BS * (q.nx + plane) * int(sizeof(CT))));
   const PatchHdr h = patch_header(q.hdr, blockIdx.x);
   // the plan data of a patch that starts later goes to L2 meanwhile (P2 tets
   // n=96 0.246 -> 0.230 ms)
@@ -291,11 +316,15 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
 #pragma unroll
     for (int e = 0; e < BS; ++e) xs[e * q.nx + i] = CT(__ldg(q.x + int64_t(e) * q.nnodes + node));
     if (i < h.nverts) {
-      double a, b, c, d;
-      ld_rec4(q.xw + 4 * size_t(node), a, b, c, d);
-      double2* v = reinterpret_cast<double2*>(vs + 4 * i);
-      v[0] = make_double2(a, b);
-      v[1] = make_double2(D == 3 ? c : 0.0, KP1 ? __ldg(q.kappa + node) : 0.0);
+      double2* v = reinterpret_cast<double2*>(vs + VS * i);
+      if constexpr (VS == 2) {
+        v[0] = __ldg(reinterpret_cast<const double2*>(q.xw + 4 * size_t(node)));
+      } else {
+        double a, b, c, d;
+        ld_rec4(q.xw + 4 * size_t(node), a, b, c, d);
+        v[0] = make_double2(a, b);
+        v[1] = make_double2(D == 3 ? c : 0.0, KP1 ? __ldg(q.kappa + node) : 0.0);
+      }
     }
   }
   if (threadIdx.x < BS) ys[threadIdx.x * plane + K * q.stride] = CT(0);
@@ -307,12 +336,16 @@ __global__ void __launch_bounds__(kPatchThreads, patch_ctas<FORM>()) k_patch_app
     CT xc[BS][K];
 #pragma unroll
     for (int a = 0; a < NB; ++a) {
-      const double2* v = reinterpret_cast<const double2*>(reinterpret_cast<const char*>(vs) + 4 * cn.off(a));
-      const double2 lo = v[0], hi = v[1];
+      const double2* v = reinterpret_cast<const double2*>(reinterpret_cast<const char*>(vs) + VS * cn.off(a));
+      const double2 lo = v[0];
       xv[a][0] = lo.x;
       xv[a][1] = lo.y;
-      if constexpr (D == 3) xv[a][2] = hi.x;
-      kap[a] = hi.y;
+      kap[a] = 0.0;
+      if constexpr (VS == 4) {
+        const double2 hi = v[1];
+        if constexpr (D == 3) xv[a][2] = hi.x;
+        kap[a] = hi.y;
+      }
     }
 #pragma unroll
     for (int j = 0; j < K; ++j) {
@@ -360,7 +393,7 @@ void run_patch_apply(const PatchPlan& B, const PatchArgs& q, cudaStream_t s) {
     auto kern = k_patch_apply<D, P, FORM, KP1, CT>;
     static unsigned long long configured = 0;
     allow_dynamic_smem(kern, configured);
-    const size_t smem = PatchPlan::pad16(uint32_t(32 * q.nv + BS * (q.nx + K * q.stride + 1) * int(sizeof(CT)))) +
+    const size_t smem = PatchPlan::pad16(uint32_t(8 * patch_vertex<D, KP1>() * q.nv + BS * (q.nx + K * q.stride + 1) * int(sizeof(CT)))) +
                         size_t(B.max_chunks) * 16;
     kern<<<unsigned(B.npatches), kPatchThreads, smem, s>>>(q);
     count_launch();
