@@ -337,10 +337,14 @@ std::unique_ptr<PatchPlan> make_patches(const Pattern& P, int max_cells) {
   return B;
 }
 
-// Cells of a patch: as many as let five 128-thread CTAs (four for elasticity)
-// share an SM.  Measured on B200 (ms per action): P2 tets n=96 0.246 with 330
-// cells (five CTAs) against 0.284 with 384 (four), 0.40 with 256; vector P2
-// elasticity n=48 0.089 with 200; P1 tets n=80 0.062 with 512, 0.066 with 768.
+// Cells of a patch, measured on B200 at two lattices (ms per action): P2 tets
+// n=96 0.246 with 330 cells (five 128-thread CTAs an SM) against 0.284 with 384
+// (four), 0.40 with 256; vector P2 elasticity n=48 0.089 with 200 (four CTAs of
+// 55 KB); P1 tets n=80 0.062 with 512, 0.066 with 768.  The cuts lie between
+// lattice planes, so the caps are met in steps: P2 tets n=96 has 324 cells in
+// every patch (1620 resident on an SM), n=40 to 90 and 63x70x57 214 to 267 on
+// average (1070 to 1340); elasticity n=48 162 (648 resident), n=30 to 47 129 to
+// 192 with CTAs of 61 to 65 KB, of which three fit (387 to 576).
 // Small meshes are cut into about 600 patches (four for each of 148 SMs), down
 // to 64 cells: one patch's latency is the action's.
 const PatchPlan& patch_plan(const Pattern& P) {
