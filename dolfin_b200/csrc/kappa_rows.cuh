@@ -17,20 +17,12 @@
 // vertex row 15 against 42, of about 165 and 110 a cell and row in all.
 #pragma once
 
-#ifndef DB2_HD
-#if defined(__CUDACC__)
-#define DB2_HD __host__ __device__ __forceinline__
-#else
-#define DB2_HD inline
-#endif
-#endif
-
 namespace db2 {
 namespace dev {
 
 // Local edges after the vertices: (2,3)(1,3)(1,2)(0,3)(0,2)(0,1) and
 // (1,2)(0,2)(0,1).
-DB2_HD void p2_kappa_edge_row(const double (&W)[2][4], const double (&k)[4], double (&o)[10]) {
+__device__ __forceinline__ void p2_kappa_edge_row(const double (&W)[2][4], const double (&k)[4], double (&o)[10]) {
   const double S = (k[0] + k[1]) + (k[2] + k[3]);
   const double u = S + k[0], w = S + k[1];
   const double u2 = 2.0 * u, w2 = 2.0 * w;
@@ -49,7 +41,7 @@ DB2_HD void p2_kappa_edge_row(const double (&W)[2][4], const double (&k)[4], dou
   o[8] = fma(W[1][2], R0, fma(W[1][0], R2, fma(W[0][2], R1, W[0][0] * P2)));
   o[9] = fma(W[1][1], R0, fma(W[1][0] + W[0][1], R1, W[0][0] * P1));
 }
-DB2_HD void p2_kappa_vertex_row(const double (&W)[1][4], const double (&k)[4], double (&o)[10]) {
+__device__ __forceinline__ void p2_kappa_vertex_row(const double (&W)[1][4], const double (&k)[4], double (&o)[10]) {
   const double S = (k[0] + k[1]) + (k[2] + k[3]);
   const double S4 = 4.0 * S;
   const double c0 = fma(20.0, k[0], S4), h = fma(8.0, k[0], -S4), v = fma(-4.0, k[0], -S);
@@ -65,7 +57,7 @@ DB2_HD void p2_kappa_vertex_row(const double (&W)[1][4], const double (&k)[4], d
   o[8] = fma(W[0][2], c0, W[0][0] * c2);
   o[9] = fma(W[0][1], c0, W[0][0] * c1);
 }
-DB2_HD void p2_kappa_edge_row(const double (&W)[2][3], const double (&k)[3], double (&o)[6]) {
+__device__ __forceinline__ void p2_kappa_edge_row(const double (&W)[2][3], const double (&k)[3], double (&o)[6]) {
   const double S = (k[0] + k[1]) + k[2];
   const double u = S + k[0], w = S + k[1];
   const double u4 = 4.0 * u, w4 = 4.0 * w;
@@ -79,7 +71,7 @@ DB2_HD void p2_kappa_edge_row(const double (&W)[2][3], const double (&k)[3], dou
   o[4] = fma(W[1][2], R0, fma(W[1][0], R2, fma(W[0][2], R1, W[0][0] * P2)));
   o[5] = fma(W[1][1], R0, fma(W[1][0] + W[0][1], R1, W[0][0] * P1));
 }
-DB2_HD void p2_kappa_vertex_row(const double (&W)[1][3], const double (&k)[3], double (&o)[6]) {
+__device__ __forceinline__ void p2_kappa_vertex_row(const double (&W)[1][3], const double (&k)[3], double (&o)[6]) {
   const double S = (k[0] + k[1]) + k[2];
   const double S3 = 3.0 * S;
   const double c0 = fma(11.0, k[0], S3), h = fma(4.0, k[0], -S), v = S + k[0];
